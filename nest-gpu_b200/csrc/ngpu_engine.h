@@ -81,6 +81,8 @@ struct Group {
   int2 *d_rec_col = nullptr;
   int *d_pin_off = nullptr;
   PoissonIn *d_pin = nullptr;
+  int *d_pin_tgt = nullptr;      // per poiss_gen edge its target (only if some neuron has several)
+  int pin_lo = 0, pin_hi = 0;    // the edges of neurons lo .. hi-1
   int *d_sg_off = nullptr, *d_sg_tidx = nullptr, *d_sg_next = nullptr;
   float *d_sg_h = nullptr;
   int lo = 0, hi = 0;            // neurons lo .. hi-1 are simulated by this process (calibration)
@@ -418,6 +420,11 @@ class Engine {
   void ensure_record_window(long long rows);
   GroupRecord group_record(Group &g);
   GroupInput group_input(Group &g);
+  PoissonMultiArgs poisson_multi_args(Group &g);
+  // the group's poiss_gen draws are made by poisson_multi_kernel, not by its update kernel
+  bool poisson_split(const Group &g) const {
+    return g.d_pin_tgt && !push_ && !(persistent && persistent_eligible());
+  }
   void run_steps(long long n);
   void run_batches_partitioned(long long n);
   int part_rank_ = 0, part_world_ = 1;
@@ -457,6 +464,7 @@ int launch_rev_arrivals(int *rev_ring, int *rev_cnt, int rev_R, int rev_cap, int
                         int k0, cudaStream_t st);
 int launch_deliver(const DeliverArgs &A, int n_blocks, int group, const Clock *clk, int k0, int M,
                    cudaStream_t st);
+int launch_poisson_multi(const PoissonMultiArgs &A, const Clock *clk, int k0, int M, cudaStream_t st);
 int launch_clock_advance(Clock *clk, int K, cudaStream_t st);
 int launch_exchange_unpack(const SpikeOut &so, const int4 *recv, int xch_cap, int world, int rank,
                            cudaStream_t st);

@@ -384,6 +384,16 @@ void Engine::calibrate() {
       g.d_pin = dalloc<PoissonIn>(pin.size());
       cuda_check(cudaMemcpy(g.d_pin_off, off.data(), (g.n + 1) * sizeof(int), cudaMemcpyHostToDevice), "pin_off");
       cuda_check(cudaMemcpy(g.d_pin, pin.data(), pin.size() * sizeof(PoissonIn), cudaMemcpyHostToDevice), "pin");
+      bool several = false;
+      for (int i = g.lo; i < g.hi; i++) several = several || off[i + 1] - off[i] > 1;
+      if (several) {
+        std::vector<int> tgt(pin.size());
+        for (int i = 0; i < g.n; i++) std::fill(tgt.begin() + off[i], tgt.begin() + off[i + 1], i);
+        g.d_pin_tgt = dalloc<int>(tgt.size());
+        cuda_check(cudaMemcpy(g.d_pin_tgt, tgt.data(), tgt.size() * sizeof(int), cudaMemcpyHostToDevice), "pin");
+        g.pin_lo = off[g.lo];
+        g.pin_hi = off[g.hi];
+      }
     }
   }
 
@@ -757,12 +767,29 @@ GroupInput Engine::group_input(Group &g) {
   in.acc = d_acc_ + g.acc_off;
   in.slot_stride = n_acc_;
   if (push_ && g.model == M_IAF_PSC_EXP) in.acc = d_pacc_ + g.acc_off;   // the delivery-at-emission ring
-  in.pin_off = g.d_pin_off;
+  in.pin_off = poisson_split(g) ? nullptr : g.d_pin_off;
   in.pin = g.d_pin;
   in.gen = d_gen_;
   in.lam_scale = (float)(dt / 1000.0);
   in.seed = kernel_seed;
   return in;
+}
+
+PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
+  const GroupInput in = group_input(g);
+  PoissonMultiArgs A;
+  A.pin = g.d_pin;
+  A.tgt = g.d_pin_tgt;
+  A.e0 = g.pin_lo;
+  A.e1 = g.pin_hi;
+  A.gen = in.gen;
+  A.acc = in.acc;
+  A.slot_stride = in.slot_stride;
+  A.n = g.n;
+  A.lam_scale = in.lam_scale;
+  A.seed = in.seed;
+  A.dt = dt;
+  return A;
 }
 
 AeifArgs Engine::aeif_args(Group &g) {
@@ -1026,6 +1053,8 @@ void Engine::launch_batch(int k0, int M, std::vector<cudaEvent_t> *ev) {
     count_launch(launch_deliver(deliver_args(), deliver_blocks_req > 0 ? deliver_blocks_req : deliver_blocks_,
                                 deliver_group, d_clk_, k0, M, stream_));
   if (ev) cuda_check(cudaEventRecord((*ev)[1], stream_), "event");
+  for (auto &g : groups_)
+    if (poisson_split(g)) count_launch(launch_poisson_multi(poisson_multi_args(g), d_clk_, k0, M, stream_));
   cudaStream_t s2 = stream_;
   if (fork) {
     cuda_check(cudaEventRecord(ev_fork_, stream_), "fork");

@@ -126,6 +126,20 @@ struct GroupInput {
   uint64_t seed;
 };
 
+// poiss_gen edges of a group drawn by a kernel of their own, before the update kernel.
+struct PoissonMultiArgs {
+  const PoissonIn *pin;
+  const int *tgt;        // per edge: target neuron, relative to its group
+  int e0, e1;            // the edges of the neurons simulated here
+  const GenPar *gen;
+  double *acc;           // slot 0 row of the group
+  size_t slot_stride;
+  int n;
+  float lam_scale;
+  uint64_t seed;
+  float dt;
+};
+
 // aeif derived parameters: uniform -> value, else a device array.
 constexpr int AEIF_NSCAL = 13;
 enum AeifPar {
