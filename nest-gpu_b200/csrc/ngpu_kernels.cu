@@ -429,6 +429,19 @@ constexpr int MAX_PAIRS = 8192;     // dspan * M
 
 typedef cub::BlockScan<int, DELIVER_THREADS> DeliverScan;
 
+// Plastic networks (one step per batch): at T mod 2^16 = 0x8000 the arrival stamps of the older
+// half become 0, at 0 those of the other half become 0x8000 (src/rev_spike.cu:93-118).  Done by
+// the step's delivery kernel, which runs before the step's plasticity kernels and reads no stamp.
+__device__ __forceinline__ void reset_stamps(const DeliverArgs &A, long long T, int block, int nblocks) {
+  const unsigned t16 = (unsigned)(T & 0xffff);
+  if (t16 != 0x8000u && t16 != 0u) return;
+  for (long long p = block * (long long)blockDim.x + threadIdx.x; p < A.n_pl; p += (long long)nblocks * blockDim.x) {
+    const unsigned short s = A.stamp[p];
+    if (t16 == 0x8000u && s >= 0x8000) A.stamp[p] = 0;
+    if (t16 == 0u && s < 0x8000) A.stamp[p] = 0x8000;
+  }
+}
+
 // The delivery of one batch by block `block` of `nblocks`; s_pref holds dspan*M+1 ints.
 template <int G, bool AGG = false, bool PF = false>
 __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock *clk, int k0, int M, int *s_pref,
@@ -436,6 +449,7 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
                                               int nblocks) {
   typedef DeliverScan Scan;
   const long long t_first = clk->tidx_base + clk->it0 + k0 + 1;   // time index of step 0
+  if (A.stamp) reset_stamps(A, t_first, block, nblocks);
   const int npairs = A.dspan * M;
   const int per = (npairs + DELIVER_THREADS - 1) / DELIVER_THREADS;
   int local = 0;

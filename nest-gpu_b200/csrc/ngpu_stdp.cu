@@ -3,7 +3,7 @@
 // Networks with plastic edges (synapse group > 0) advance one time step per batch, and
 // each step T runs, around the step's delivery and update kernels:
 //   before:  stamp reset at the 16-bit wrap points (src/nestgpu.cu:490-498,
-//            src/rev_spike.cu:93-118);
+//            src/rev_spike.cu:93-118), by the delivery kernel (reset_stamps);
 //   after:   forward pass over the spikes arriving in T: each plastic edge records T as
 //            its last arrival and is depressed against its target's last spike
 //            (src/get_spike.cu:85-95); then the reverse pass: the plastic in-edges of
@@ -14,6 +14,8 @@
 // (src/syn_model.cu:43-56): STDPUpdate (src/stdp.cu:36-64) in FP64, or the linear test
 // model (src/test_syn_model.cu:35-40).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "ngpu_aeif.cuh"
 #include "ngpu_types.h"
@@ -44,35 +46,40 @@ __device__ __forceinline__ long long step_tidx(const Clock *clk, int k0) {
   return clk->tidx_base + clk->it0 + k0 + 1;
 }
 
-// Up at T mod 2^16 = 0x8000: stamps of the older half become 0; down at 0: stamps of the
-// other half become 0x8000.
-__global__ void stdp_stamp_reset_kernel(const StdpArgs A, const Clock *clk, int k0) {
-  const unsigned t16 = (unsigned)(step_tidx(clk, k0) & 0xffff);
-  if (t16 != 0x8000u && t16 != 0u) return;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < A.n_pl;
-       p += (long long)gridDim.x * blockDim.x) {
-    const unsigned short s = A.stamp[p];
-    if (t16 == 0x8000u && s >= 0x8000) A.stamp[p] = 0;
-    if (t16 == 0u && s < 0x8000) A.stamp[p] = 0x8000;
-  }
+// One plastic edge, as one 16-byte load.
+__device__ __forceinline__ PlasticEdge ldg_plastic(const PlasticEdge *p) {
+  static_assert(sizeof(PlasticEdge) == 16, "PlasticEdge is one 16-byte word");
+  const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+  PlasticEdge e;
+  e.pos = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+  e.target = (int)v.z;
+  e.group = (int)v.w;
+  return e;
 }
 
-// One warp per delay group: its lanes take the spikes emitted T-1-(dmin+dd) steps ago.
-__global__ void stdp_forward_kernel(const StdpArgs A, const Clock *clk, int k0) {
-  const int dd = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (dd >= A.dspan) return;
+// Both passes are latency chains (ring or spike flag -> segment -> edge -> weight, then FP64
+// exp and pow) over a few thousand edges, so what counts is how many edges run side by side:
+// a warp per (spike, delay group) here, the warps of a block over the in-edges of its spiking
+// targets below.  4000 neurons, 100 in-edges each, 24 spikes a step: with one thread per spike
+// and one per target, each walking its edges, 24 and 137 us; now the two, the delivery and the
+// update together take 16.9 us a step (173 before).
+__global__ void __launch_bounds__(256) stdp_forward_kernel(const StdpArgs A, const Clock *clk, int k0) {
+  pdl_enter();
+  const int dd = blockIdx.x;
   const long long T = step_tidx(clk, k0);
-  const long long te = T - 1 - (A.dmin + dd);
+  const long long te = T - 1 - (A.dmin + dd);   // the delay group's emission step
   if (te < 1) return;
   const int rs = (int)(te % A.R);
   int cnt = A.ring_cnt[rs];
   cnt = cnt < A.cap ? cnt : A.cap;
   const unsigned short t16 = (unsigned short)(T & 0xffff);
-  for (int j = threadIdx.x & 31; j < cnt; j += 32) {
+  const int lane = threadIdx.x & 31, nw = (int)(gridDim.y * (blockDim.x >> 5));
+  for (int j = (int)(blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)); j < cnt; j += nw) {
     const int src = A.ring[(size_t)rs * A.cap + j].x;
     const size_t key = (size_t)src * A.dspan + dd;
-    for (int p = A.pl_off[key]; p < A.pl_off[key + 1]; p++) {
-      const PlasticEdge e = A.pl[p];
+    const int p1 = __ldg(A.pl_off + key + 1);
+    for (int p = __ldg(A.pl_off + key) + lane; p < p1; p += 32) {
+      const PlasticEdge e = ldg_plastic(A.pl + p);
       A.stamp[p] = t16;
       const int last = A.last_tidx[e.target];
       if (last < 0) continue;   // the target has not spiked yet
@@ -86,20 +93,42 @@ __global__ void stdp_forward_kernel(const StdpArgs A, const Clock *clk, int k0) 
   }
 }
 
-__global__ void stdp_reverse_kernel(const StdpArgs A, const Clock *clk, int k0) {
+// A block serves 32 targets with plastic in-edges; its eight warps share the 32-edge chunks of
+// those that spiked in step T.
+constexpr int REV_TARGETS = 32;
+
+__global__ void __launch_bounds__(256) stdp_reverse_kernel(const StdpArgs A, const Clock *clk, int k0) {
+  pdl_enter();
   const long long T = step_tidx(clk, k0);
   const unsigned short t16 = (unsigned short)(T & 0xffff);
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < A.n_rev_nodes; r += gridDim.x * blockDim.x) {
-    if ((long long)A.last_tidx[A.rev_node[r]] != T) continue;
-    for (int q = A.rev_off[r]; q < A.rev_off[r + 1]; q++) {
-      const int p = A.rev_id[q];
-      const unsigned short Dt_int = (unsigned short)(t16 - A.stamp[p]);
-      if (Dt_int < MAX_SYN_DT) {
-        const PlasticEdge e = A.pl[p];
-        const int g = e.group - 1;
-        float &w = A.edge[e.pos].w;
-        w = synapse_update(A.syn_type[g], A.syn_par + g * SYN_NPAR, w, A.dt * (float)Dt_int);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (long long r0 = (long long)blockIdx.x * REV_TARGETS; r0 < A.n_rev_nodes; r0 += (long long)gridDim.x * REV_TARGETS) {
+    const int r = (int)r0 + lane;
+    int q0 = 0, q1 = 0;
+    bool spiked = false;
+    if (r < A.n_rev_nodes) {
+      q0 = __ldg(A.rev_off + r);
+      q1 = __ldg(A.rev_off + r + 1);
+      spiked = (long long)A.last_tidx[__ldg(A.rev_node + r)] == T;
+    }
+    int chunk = 0;             // chunks of the block's spiking targets so far
+    for (unsigned mask = __ballot_sync(0xffffffffu, spiked); mask; mask &= mask - 1) {
+      const int f = __ffs(mask) - 1;
+      const int a = __shfl_sync(0xffffffffu, q0, f), b = __shfl_sync(0xffffffffu, q1, f);
+      const int nc = (b - a + 31) >> 5;
+      for (int c = ((warp - chunk) % nw + nw) % nw; c < nc; c += nw) {
+        const int q = a + 32 * c + lane;
+        if (q >= b) continue;
+        const int p = __ldg(A.rev_id + q);
+        const unsigned short Dt_int = (unsigned short)(t16 - A.stamp[p]);
+        if (Dt_int < MAX_SYN_DT) {
+          const PlasticEdge e = ldg_plastic(A.pl + p);
+          const int g = e.group - 1;
+          float &w = A.edge[e.pos].w;
+          w = synapse_update(A.syn_type[g], A.syn_par + g * SYN_NPAR, w, A.dt * (float)Dt_int);
+        }
       }
+      chunk += nc;
     }
   }
 }
@@ -110,6 +139,7 @@ __global__ void stdp_reverse_kernel(const StdpArgs A, const Clock *clk, int k0) 
 // slot is emptied for T + rev_R.
 __global__ void rev_arrival_kernel(int *rev_ring, int *rev_cnt, int rev_R, int rev_cap, int *last_rev,
                                    const Clock *clk, int k0) {
+  pdl_enter();
   const long long T = step_tidx(clk, k0);
   const int rs = (int)(T % rev_R);
   int cnt = rev_cnt[rs];
@@ -121,24 +151,20 @@ __global__ void rev_arrival_kernel(int *rev_ring, int *rev_cnt, int rev_R, int r
 
 int launch_rev_arrivals(int *rev_ring, int *rev_cnt, int rev_R, int rev_cap, int *last_rev, const Clock *clk,
                         int k0, cudaStream_t st) {
-  rev_arrival_kernel<<<1, 256, 0, st>>>(rev_ring, rev_cnt, rev_R, rev_cap, last_rev, clk, k0);
-  return 1;
-}
-
-int launch_stdp_reset(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st) {
-  const long long nb = (A.n_pl + 255) / 256;
-  stdp_stamp_reset_kernel<<<(int)(nb < 148 * 8 ? (nb > 0 ? nb : 1) : 148 * 8), 256, 0, st>>>(A, clk, k0);
+  launch_k(rev_arrival_kernel, dim3(1), dim3(256), 0, st, rev_ring, rev_cnt, rev_R, rev_cap, last_rev, clk, k0);
   return 1;
 }
 
 int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st) {
-  stdp_forward_kernel<<<(A.dspan + 3) / 4, 128, 0, st>>>(A, clk, k0);
+  // up to eight blocks (64 warps) per delay group while the grid stays below four blocks per SM
+  const int y = std::max(1, std::min(8, 592 / A.dspan));
+  launch_k(stdp_forward_kernel, dim3(A.dspan, y), dim3(256), 0, st, A, clk, k0);
   return 1;
 }
 
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st) {
-  const int nb = (A.n_rev_nodes + 127) / 128;
-  stdp_reverse_kernel<<<nb < 148 * 8 ? (nb > 0 ? nb : 1) : 148 * 8, 128, 0, st>>>(A, clk, k0);
+  const int nb = (A.n_rev_nodes + REV_TARGETS - 1) / REV_TARGETS;
+  launch_k(stdp_reverse_kernel, dim3(std::max(1, std::min(nb, 148 * 32))), dim3(256), 0, st, A, clk, k0);
   return 1;
 }
 

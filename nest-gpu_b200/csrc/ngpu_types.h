@@ -267,6 +267,8 @@ struct DeliverArgs {
   int aggregate;         // 1 (with 32-lane groups): warp-aggregated reductions
   int prefetch;          // 1: the next work item's ring entry and offsets loaded ahead
   int4 *xch;             // partitioned network: exchange buffer whose count the batch clears
+  unsigned short *stamp; // plastic networks: arrival stamps [n_pl], reset at their wrap points
+  long long n_pl;
 };
 
 // Plastic edge (synapse group > 0): its position in the delivery CSR, its target node and
