@@ -87,14 +87,8 @@ __device__ __forceinline__ StepT step_at(const Clock &c, int k0, int m, float dt
   return s;
 }
 
-// PushSpike (src/spike_buffer.cu:162-242) on the ring design.  RING = false (delivery at
-// emission): the spike goes to no ring, its out-edges are added by the caller.
-template <bool RING = true>
-__device__ __forceinline__ void push_spike(const SpikeOut &so, const GroupSpikeRec &rec, int node,
-                                           int rel, float height, long long tidx, double tnow) {
-  so.last_tidx[node] = (int)tidx;
-  so.last_height[node] = height;
-  atomicAdd(so.n_spikes, 1ULL);
+// The group's own spike records: its counter and recorded times.
+__device__ __forceinline__ void file_spike(const SpikeOut &so, const GroupSpikeRec &rec, int rel, double tnow) {
   if (rec.spike_count) rec.spike_count[rel] += 1;
   if (rec.n_rec) {
     int nr = rec.n_rec[rel];
@@ -105,6 +99,17 @@ __device__ __forceinline__ void push_spike(const SpikeOut &so, const GroupSpikeR
       atomicOr(so.status, ST_REC_TIMES_FULL);
     }
   }
+}
+
+// PushSpike (src/spike_buffer.cu:162-242) on the ring design.  RING = false (delivery at
+// emission): the spike goes to no ring, its out-edges are added by the caller.
+template <bool RING = true>
+__device__ __forceinline__ void push_spike(const SpikeOut &so, const GroupSpikeRec &rec, int node,
+                                           int rel, float height, long long tidx, double tnow) {
+  so.last_tidx[node] = (int)tidx;
+  so.last_height[node] = height;
+  atomicAdd(so.n_spikes, 1ULL);
+  file_spike(so, rec, rel, tnow);
   if (so.last_rev) {
     // the spike reaches the node's own synapses (STDP) now or den_delay steps later
     // (src/spike_buffer.cu:183-186, 279-281, 314-316)

@@ -138,7 +138,7 @@ class Engine {
                                   // (set before calibration)
   int update_occupancy = 0;       // 1: register-capped aeif update kernel
   int update_trial_iter = 0;      // 1: aeif update kernel advances one RK5 trial per iteration
-  int persistent = 0;             // iaf-only networks: persistent cooperative step loop
+  int persistent = -1;            // iaf-only networks: persistent cooperative step loop (-1: by persistent_auto)
   int launch_pdl = -1;            // programmatic dependent launch of the batch kernels (-1: one-step batches)
   int barrier_extra = 0;          // test hook: blocks the persistent loop's barriers wait for in excess
   bool use_device_rng = true;     // cuRAND device generator (as the reference) if a GPU exists
@@ -408,7 +408,10 @@ class Engine {
   int n_iaf_multi_ = 0, iaf_multi_blocks_ = 0;
   void prepare_multi();
   bool persistent_eligible() const;
+  bool persistent_auto(long long steps) const;
+  int pers_blocks_ = 0;          // blocks of the persistent loop (0: it cannot run this network)
   bool push_eligible() const;
+  bool iaf_only() const;
   void run_persistent(int steps);
 
   template <class T> T *dalloc(size_t n);
@@ -423,7 +426,7 @@ class Engine {
   PoissonMultiArgs poisson_multi_args(Group &g);
   // the group's poiss_gen draws are made by poisson_multi_kernel, not by its update kernel
   bool poisson_split(const Group &g) const {
-    return g.d_pin_tgt && !push_ && !(persistent && persistent_eligible());
+    return g.d_pin_tgt && !push_ && !(persistent > 0 && persistent_eligible());
   }
   void run_steps(long long n);
   void run_batches_partitioned(long long n);
@@ -476,9 +479,10 @@ double measure_random_reduction_rate(size_t bytes, long long n_ops);
 // STDP (ngpu_stdp.cu)
 int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
-int launch_persistent_iaf(const DeliverArgs &D, int group, const IafArgs *tab, const int *first, int ngroups,
-                          const SpikeOut &so, const Clock *clk, int steps, int M, GridBarrier *bar, int max_blocks,
-                          int barrier_extra, cudaStream_t st);
+int persistent_blocks(int total_n, int dspan);
+int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
+                          const Clock *clk, int steps, GridBarrier *bar, uint64_t seed, int nblocks, int barrier_extra,
+                          cudaStream_t st);
 int deliver_max_pairs();
 void pack_delivery_csr_noalloc(const int *src, const int *dly, const unsigned *target, const float *weight,
                                size_t n, int n_nodes, int dspan, unsigned long long *seg_off, EdgeW *edge,

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "ngpu_aeif.cuh"
+#include "ngpu_iaf.cuh"
 #include "ngpu_math.cuh"
 #include "ngpu_types.h"
 
@@ -25,14 +26,6 @@ namespace ngpu {
 
 bool g_launch_pdl = false;
 void set_launch_pdl(bool on) { g_launch_pdl = on; }
-
-// ---------------------------------------------------------------------------
-// iaf_psc_exp exact propagator (src/iaf_psc_exp.cu:85-110)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float iget(const IafArgs &A, int j, int i) {
-  const float *p = A.parr[j];
-  return p ? __ldg(p + i) : A.pval[j];
-}
 
 // Delivery at emission: the block adds the out-edges of node `src`, which spiked at time
 // index `tidx`, into the accumulator ring.  The source's edges are contiguous in the CSR,
@@ -84,12 +77,8 @@ __device__ __noinline__ unsigned long long push_out_edges(const PushOut &po, int
 __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so, const Clock *clk, int k0,
                                            int M, int i) {
   const int n = A.n;
-  float Iex = A.var[i], Iin = A.var[(size_t)n + i], V = A.var[2 * (size_t)n + i],
-        refr = A.var[3 * (size_t)n + i];
-  const float I_e = iget(A, IP_I_e, i), P20 = iget(A, IP_P20, i), P21ex = iget(A, IP_P21ex, i),
-              P21in = iget(A, IP_P21in, i), P22 = iget(A, IP_P22, i), P11ex = iget(A, IP_P11ex, i),
-              P11in = iget(A, IP_P11in, i), theta = iget(A, IP_Theta_rel, i),
-              V_reset = iget(A, IP_V_reset_rel, i), refr_steps = iget(A, IP_refr_steps, i);
+  IafRegs q;
+  iaf_load(A, i, q);
   const Clock cl = *clk;
   const long long rec_it0 = cl.rec_it0;
   PoissonCache pc;
@@ -98,31 +87,16 @@ __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so,
     const StepT t = step_at(cl, k0, m, A.dt);
     double apf[2];
     acc_prefetch<2>(apf, 2, n, i, A.in, m);
-    if (refr > 0.0f) {
-      refr = __fsub_rn(refr, 1.0f);
-    } else {
-      V = __fmaf_rn(I_e, P20, __fmaf_rn(Iin, P21in, __fmaf_rn(Iex, P21ex, __fmul_rn(V, P22))));
-    }
-    Iex = __fmul_rn(Iex, P11ex);
-    Iin = __fmul_rn(Iin, P11in);
-    if (V >= theta) {
-      push_spike(so, A.srec, A.i0 + i, i, 1.0f, t.tidx, t.tnow);
-      V = V_reset;
-      refr = refr_steps;
-    }
+    if (iaf_step(q)) push_spike(so, A.srec, A.i0 + i, i, 1.0f, t.tidx, t.tnow);
     if (A.rec.first) {
-      const float yr[4] = {Iex, Iin, V, refr};
-      write_records<4>(A.rec, so, A.i0 + i, i, yr, 4, refr, t.it - rec_it0, t.tidx);
+      const float yr[4] = {q.Iex, q.Iin, q.V, q.refr};
+      write_records<4>(A.rec, so, A.i0 + i, i, yr, 4, q.refr, t.it - rec_it0, t.tidx);
     }
     double in[2];
     step_inputs_pf<2>(in, apf, 2, n, i, A.in, pc, m, t.tidx, t.tnow);
-    if (in[0] != 0.0) Iex = (float)__fma_rn(in[0], 1.0, (double)Iex);
-    if (in[1] != 0.0) Iin = (float)__fma_rn(in[1], 1.0, (double)Iin);
+    iaf_fold(q, in);
   }
-  A.var[i] = Iex;
-  A.var[(size_t)n + i] = Iin;
-  A.var[2 * (size_t)n + i] = V;
-  A.var[3 * (size_t)n + i] = refr;
+  iaf_store(A, i, q);
 }
 
 // iaf_neuron with delivery at emission: every thread of the block runs the loop (`valid` false
@@ -594,100 +568,6 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_batch_kernel(const De
 __global__ void clock_advance_kernel(Clock *clk, int K) {
   pdl_enter();
   clk->it0 += K;
-}
-
-// ---------------------------------------------------------------------------
-// Persistent step loop for networks whose neurons are all iaf_psc_exp.  One
-// cooperative launch (all blocks co-resident) advances K steps in batches of M:
-// delivery, grid barrier, update of every population, grid barrier.  With a minimum
-// delay of one step (M = 1) this replaces two launches per step.
-// ---------------------------------------------------------------------------
-// Counting barrier over the blocks of the launch.  Waits are bounded: after 2^24 polls
-// a block records a timeout in the status word, and every later barrier of the launch
-// returns false at once, so the kernel ends instead of waiting for ever.
-__device__ __forceinline__ bool grid_barrier(GridBarrier *bar, unsigned nblocks, unsigned *status) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = (((volatile unsigned *)status)[0] & ST_BARRIER_TIMEOUT) ? 0 : 1;
-    if (ok) {
-      const unsigned g = ((volatile unsigned *)&bar->gen)[0];
-      __threadfence();
-      if (atomicAdd(&bar->count, 1u) + 1u == nblocks) {
-        atomicExch(&bar->count, 0u);
-        __threadfence();
-        atomicAdd(&bar->gen, 1u);
-      } else {
-        long long polls = 0;
-        while (((volatile unsigned *)&bar->gen)[0] == g) {
-          if (++polls > (1LL << 24)) {
-            atomicOr(status, ST_BARRIER_TIMEOUT);
-            ok = 0;
-            break;
-          }
-          __nanosleep(64);
-        }
-      }
-      __threadfence();
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-template <int G>
-__global__ void __launch_bounds__(DELIVER_THREADS) persistent_iaf_kernel(
-    const DeliverArgs D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut so, const Clock *clk,
-    int K, int M, GridBarrier *bar, int extra) {
-  extern __shared__ int s_pref[];
-  __shared__ typename DeliverScan::TempStorage scan_tmp;
-  const int total_n = first[ngroups];
-  const unsigned nb = gridDim.x + (unsigned)extra;   // extra > 0 only in the timeout test
-  for (int k0 = 0; k0 < K; k0 += M) {
-    const int mb = (K - k0 < M) ? K - k0 : M;
-    deliver_batch<G>(D, clk, k0, mb, s_pref, scan_tmp, blockIdx.x, gridDim.x);
-    if (!grid_barrier(bar, nb, so.status)) return;
-    for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < total_n; gi += gridDim.x * blockDim.x) {
-      int lo = 0, hi = ngroups;   // group with first[g] <= gi < first[g+1]
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (first[mid] <= gi) lo = mid; else hi = mid;
-      }
-      iaf_neuron(tab[lo], so, clk, k0, mb, gi - first[lo]);
-    }
-    if (!grid_barrier(bar, nb, so.status)) return;
-  }
-}
-
-// Cooperative launch of the persistent loop over `steps` steps; the grid is the number of
-// blocks that fit on the GPU at once (at most `max_blocks`).
-int launch_persistent_iaf(const DeliverArgs &D, int group, const IafArgs *tab, const int *first, int ngroups,
-                          const SpikeOut &so, const Clock *clk, int steps, int M, GridBarrier *bar, int max_blocks,
-                          int barrier_extra, cudaStream_t st) {
-  const size_t smem = (size_t)(D.dspan * M + 1) * sizeof(int);
-  void *fn = group == 8 ? (void *)persistent_iaf_kernel<8>
-                        : group == 16 ? (void *)persistent_iaf_kernel<16> : (void *)persistent_iaf_kernel<32>;
-  int dev = 0, n_sm = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, DELIVER_THREADS, smem);
-  int nblocks = n_sm * per_sm;
-  if (max_blocks > 0 && nblocks > max_blocks) nblocks = max_blocks;
-  if (nblocks < 1) return -1;
-  DeliverArgs d = D;
-  const IafArgs *t = tab;
-  const int *f = first;
-  int ng = ngroups;
-  SpikeOut s = so;
-  const Clock *c = clk;
-  int k = steps, m = M;
-  GridBarrier *b = bar;
-  int x = barrier_extra;
-  void *args[] = {&d, &t, &f, &ng, &s, &c, &k, &m, &b, &x};
-  if (cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(DELIVER_THREADS), args, smem, st) != cudaSuccess)
-    return -1;
-  return 1;
 }
 
 // ---------------------------------------------------------------------------

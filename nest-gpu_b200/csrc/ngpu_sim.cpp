@@ -405,8 +405,12 @@ void Engine::calibrate() {
   // synaptic spikes of the same step (src/nestgpu.cu:469-635 order)
   if (plastic_) batch_ = 1;
   if (dspan_ * batch_ > deliver_max_pairs()) batch_ = std::max(1, deliver_max_pairs() / dspan_);
-  d_acc_ = dalloc<double>(n_acc_ * batch_);
-  cuda_check(cudaMemset(d_acc_, 0, std::max<size_t>(n_acc_ * batch_, 1) * sizeof(double)), "memset");
+  // (the persistent loop of an iaf-only network has the arrivals of four steps open at a time)
+  pers_blocks_ = 0;
+  if (iaf_only()) pers_blocks_ = persistent_blocks(N, dspan_);
+  const size_t acc_slots = pers_blocks_ ? std::max(batch_, 4) : batch_;
+  d_acc_ = dalloc<double>(n_acc_ * acc_slots);
+  cuda_check(cudaMemset(d_acc_, 0, std::max<size_t>(n_acc_ * acc_slots, 1) * sizeof(double)), "memset");
   // delivery at emission: a spike of step t reaches steps t + 1 + dmin .. t + dmin + dspan,
   // all after its batch (batch_ <= dmin + 1); the ring has one slot per step of that reach
   // and of the batch being read, so a slot being read is never one being written
@@ -1119,22 +1123,32 @@ void Engine::prepare_multi() {
 }
 
 // The persistent step loop serves networks whose only neurons are iaf_psc_exp groups
-// (Poisson generators have no kernel of their own).
-bool Engine::persistent_eligible() const {
-  if (plastic_ || part_world_ > 1 || push_) return false;
-  bool any = false;
-  for (auto &g : groups_) {
-    if (g.n <= 0 || g.model == M_POISS_GEN) continue;
-    if (g.model != M_IAF_PSC_EXP) return false;
-    any = true;
-  }
-  return any;
+// (Poisson generators have no kernel of their own) and that fit it.
+bool Engine::persistent_eligible() const { return !push_ && pers_blocks_ > 0; }
+
+// Networks with a minimum delay of one step run in the persistent loop by themselves: a step is
+// then two short dependent launches otherwise (ngpu_persist.cu has both times).  With longer
+// minimum delays the per-batch kernels spread their launches over several steps and need no
+// barrier per step (3.5 us a step at 15-step batches, 12,500 neurons, 42k events a step).
+// A call costs a table upload, the first step's delivery from the ring and an extra barrier:
+// calls of 1, 2, 4, 8 and 16 steps took 78, 81, 84, 99 and 123 us on the microcircuit at a tenth
+// of its size (79, 85, 92, 110 and 142 us at full size) against 50, 63, 95, 149 and 267 us (54, 72,
+// 109, 184 and 337 us) per batch, so the line lies at four steps.  Neurons with several
+// generators each stay with the per-batch kernels, where poisson_multi_kernel spreads their draws
+// over the GPU.
+bool Engine::persistent_auto(long long steps) const {
+  if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < 4) return false;
+  for (auto &g : groups_)
+    if (g.d_pin_tgt) return false;
+  return true;
 }
 
-// Delivery at emission serves the same networks as the persistent loop: iaf_psc_exp groups
-// only (their spikes have height 1 and their kernel is the only spike source), no plastic
-// edges, one process.
-bool Engine::push_eligible() const {
+// Delivery at emission serves the same networks as the persistent loop.
+bool Engine::push_eligible() const { return iaf_only(); }
+
+// iaf_psc_exp groups only (their spikes have height 1 and their kernel is the only spike
+// source), no plastic edges, one process.
+bool Engine::iaf_only() const {
   if (plastic_ || part_world_ > 1) return false;
   bool any = false;
   for (auto &g : groups_) {
@@ -1148,9 +1162,8 @@ bool Engine::push_eligible() const {
 // `steps` steps in one cooperative launch of the persistent loop, then the clock advance.
 void Engine::run_persistent(int steps) {
   cuda_check(cudaMemsetAsync(d_bar_, 0, sizeof(GridBarrier), stream_), "barrier reset");
-  const int r = launch_persistent_iaf(deliver_args(), deliver_group, d_iaf_tab_, d_iaf_first_, n_iaf_multi_,
-                                      spike_out(), d_clk_, steps, batch_, d_bar_,
-                                      deliver_blocks_req > 0 ? deliver_blocks_req : 0, barrier_extra, stream_);
+  const int r = launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_,
+                                      steps, d_bar_, kernel_seed, pers_blocks_, barrier_extra, stream_);
   if (r < 0) throw NgpuError(std::string("cooperative launch of the persistent step loop failed: ") +
                              cudaGetErrorString(cudaGetLastError()));
   launch_clock_advance(d_clk_, steps, stream_);
@@ -1213,6 +1226,9 @@ void Engine::run_batches_partitioned(long long n) {
   }
 }
 
+// Steps per launch of the persistent loop: launch and prologue are a few steps' time.
+constexpr long long PERS_STEPS = 2000;
+
 void Engine::run_steps(long long n) {
   if (part_world_ > 1) {
     run_batches_partitioned(n);
@@ -1226,19 +1242,20 @@ void Engine::run_steps(long long n) {
     window = std::min<long long>(n, REC_WINDOW);
     ensure_record_window(window);
   }
-  const bool pers = persistent && persistent_eligible();
+  const bool pers = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(n));
   if (pers) prepare_multi();
   long long done = 0;
   while (done < n) {
     const long long w = std::min(window, n - done);
     long long left = w;
     while (left > 0) {
-      const int steps = (int)std::min<long long>(K, left);
       if (pers) {
+        const int steps = (int)std::min<long long>(PERS_STEPS, left);
         run_persistent(steps);
         left -= steps;
         continue;
       }
+      const int steps = (int)std::min<long long>(K, left);
       auto itg = graphs_.find(steps);
       if (itg == graphs_.end()) {
         prepare_multi();
@@ -1332,6 +1349,7 @@ void Engine::check_status() {
     cuda_check(cudaMemcpy(d_status_, &keep, sizeof(unsigned), cudaMemcpyHostToDevice), "status");
     status_seen_ &= ~ST_BARRIER_TIMEOUT;
     persistent = 0;
+    cuda_check(cudaMemset(d_acc_, 0, n_acc_ * (size_t)std::max(batch_, 4) * sizeof(double)), "memset");
     throw NgpuError("a grid barrier of the persistent step loop timed out; the simulation state is invalid "
                     "(the engine falls back to per-batch launches)");
   }

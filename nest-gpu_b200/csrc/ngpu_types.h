@@ -38,8 +38,7 @@ enum Status : unsigned {
 
 // Barrier state of the persistent step loop (device memory, zero-initialised).
 struct GridBarrier {
-  unsigned count;        // blocks arrived at the current barrier
-  unsigned gen;          // barriers completed
+  unsigned count;        // arrivals since the launch
 };
 
 // Simulation clock in device memory.  A CUDA graph covers a fixed number of steps

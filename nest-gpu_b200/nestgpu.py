@@ -1449,9 +1449,9 @@ def SetUpdateThreads(n):
 
 
 def SetPersistent(on=True):
-    """iaf_psc_exp-only networks: run the steps in one cooperative launch per graph's worth
-    of steps, or in per-batch launches captured in CUDA graphs (the default; engine
-    extension)."""
+    """iaf_psc_exp-only networks: run the steps in a persistent cooperative launch (True) or in
+    per-batch launches captured in CUDA graphs (False).  Without a call the engine chooses: the
+    persistent loop for minimum delays of one step (engine extension)."""
     _need_b200("SetPersistent")
     return _check(_c["NGPU_SetPersistent"](1 if on else 0))
 

@@ -1,0 +1,126 @@
+"""The persistent step loop of iaf_psc_exp networks against the oracle and the per-batch kernels,
+bit for bit: neuron counts around the blocks and at the loop's capacity, delay ranges from one
+step to its largest number of delay groups (first total delays of one, two and more steps, which
+take different paths), calls of one, two and three steps, and turns between the two forms."""
+import numpy as np
+import pytest
+
+import nestgpu as ngpu
+import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def fresh_engine():
+    ngpu.Reset()
+    ngpu.SetVerbosityLevel(0)
+    yield
+    ngpu.Reset()
+
+
+def _net(api, n, lo, hi, k=20):
+    """Two populations of about n / 3 and 2 n / 3 neurons, delays lo .. hi ms."""
+    api.SetKernelStatus("rnd_seed", 5)
+    na = max(1, n // 3)
+    a = api.Create("iaf_psc_exp", na)
+    b = api.Create("iaf_psc_exp", max(1, n - na))
+    api.SetStatus(b, {"tau_ex": 0.7, "I_e": 300.0})
+    pg = api.Create("poisson_generator", 2)
+    api.SetStatus(pg, "rate", 9000.0)
+    api.SetStatus([pg[1]], {"start": 2.0, "stop": 14.0})
+    api.Connect([pg[0]], a, {"rule": "all_to_all"}, {"weight": 60.0, "delay": 1.0, "receptor": 0})
+    api.Connect([pg[1]], b, {"rule": "all_to_all"}, {"weight": 60.0, "delay": 1.0, "receptor": 0})
+    for s, src in enumerate((a, b)):
+        for t, tgt in enumerate((a, b)):
+            api.ConnectFixedIndegreeGPU(src, tgt, k, 20.0 if s == 0 else -15.0, lo, hi, receptor=s, seed=10 + 2 * s + t)
+    api.ActivateSpikeCount(a)
+    api.ActivateSpikeCount(b)
+    return a, b
+
+
+def _state(api, pops):
+    return (np.concatenate([np.asarray(api.GetStatus(p, "spike_count")).ravel() for p in pops]),
+            np.concatenate([np.asarray(api.GetStatus(p, "V_m_rel"), dtype=np.float32).ravel() for p in pops]))
+
+
+@pytest.mark.parametrize("n,lo,hi", [(2, 0.1, 0.1), (147, 0.1, 0.2), (149, 0.1, 3.0), (1000, 0.2, 0.2), (1000, 0.2, 1.7),
+                                     (700, 0.3, 2.0), (300, 1.5, 1.5), (900, 0.1, 25.6)])
+def test_delay_ranges_match_oracle(n, lo, hi):
+    ngpu.SetPersistent(True)
+    pops = _net(ngpu, n, lo, hi)
+    o = orc.Oracle()
+    opops = _net(o, n, lo, hi)
+    for t in (20.0, 0.1, 0.2, 0.3, 13.7):
+        ngpu.Simulate(t)
+        o.Simulate(t)
+    c, v = _state(ngpu, pops)
+    co, vo = _state(o, opops)
+    assert co.sum() > 0 and np.array_equal(c, co)
+    assert np.array_equal(v, vo)
+    assert ngpu.GetStats()["n_events"] == o.NEvents() and ngpu.GetStats()["status"] == 0
+
+
+@pytest.mark.parametrize("n,hi", [(576 * 148, 1.0), (576 * 148 + 1, 1.0), (400, 25.7)])
+def test_capacity_and_what_lies_beyond_it(n, hi):
+    """The largest network of the loop, one neuron more, and one delay group too many (the last
+    two run in the per-batch kernels) equal the per-batch kernels."""
+    res = []
+    for pers in (True, False):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        ngpu.SetPersistent(pers)
+        pops = _net(ngpu, n, 0.1, hi, k=5)
+        ngpu.Simulate(12.0)
+        res.append(_state(ngpu, pops) + (ngpu.GetStats()["n_events"],))
+    assert res[0][0].sum() > 0 and all(np.array_equal(x, y) for x, y in zip(*res))
+
+
+def test_turns_between_the_forms():
+    """Persistent calls, per-batch calls, single steps and short calls of the automatic choice,
+    spikes in flight at every change, give what the per-batch kernels alone give."""
+    def run(modes):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 500, 0.1, 2.9)
+        for m in modes:
+            ngpu.SetPersistent(m)
+            ngpu.Simulate(4.0)
+            for _ in range(3):
+                ngpu.SimulationStep()
+            ngpu.EndSimulation()
+            ngpu.Simulate(0.7)
+        return _state(ngpu, pops) + (ngpu.GetStats()["n_events"],)
+    want = run([False] * 4)
+    assert want[0].sum() > 100
+    for modes in ([True] * 4, [True, False, True, False]):
+        assert all(np.array_equal(x, y) for x, y in zip(run(modes), want))
+
+
+def test_two_networks_in_two_threads():
+    """Two host threads run a network each at the same time (one engine per thread): their
+    persistent launches share the GPU and the results are those of a network alone."""
+    import threading
+
+    def run(out, key):
+        ngpu.SetOnException(1)     # error handling is per thread
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 800 + key, 0.1, 2.0)
+        for _ in range(20):
+            ngpu.Simulate(5.0)
+        out[key] = _state(ngpu, pops)
+        ngpu.Reset()
+
+    alone, both = {}, {}
+    for key in (0, 1):
+        t = threading.Thread(target=run, args=(alone, key))
+        t.start()
+        t.join()
+    threads = [threading.Thread(target=run, args=(both, key)) for key in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for key in (0, 1):
+        assert alone[key][0].sum() > 0
+        assert all(np.array_equal(x, y) for x, y in zip(alone[key], both[key]))
