@@ -384,6 +384,10 @@ int NGPU_SetPersistent(int on);
    (default) uses it for batches of one time step only (a minimum delay of one step), where a
    step is two short launches.  The autotuner tries both.  No counterpart in the reference. */
 int NGPU_SetProgrammaticLaunch(int on);
+/* Test hook: number of inputs on which the engine's branch-free reciprocal and quotient differ
+   from the correctly rounded ones (0), over the whole range in which they are used. */
+long long NGPU_TestRoundedOps();
+
 /* Test hook for the failure path of the persistent loop: with extra > 0 its grid barriers wait
    for more blocks than the launch has, so each wait runs out after its bounded number of polls
    (a second or two); the kernel records the timeout and returns, and the Simulate call fails

@@ -471,13 +471,39 @@ __device__ __forceinline__ void rk5_begin(const float *y, float h, const AeifQ<M
   constexpr int NVM = 2 + AeifShape<MODEL>::npv * PMAX;
   const int NV = 2 + AeifShape<MODEL>::npv * q.ports();
   aeif_derivs(y, k1, q, refr);
+  bool normal = true;
 #pragma unroll
   for (int i = 0; i < NVM; i++) {
     if (i < NV) {
-      float ys = __fadd_rn(__fadd_rn(fabsf(y[i]), fabsf(__fmul_rn(k1[i], h))), ck::scal_min);
-      iys[i] = __fdiv_rn(1.0f, ys);
+      iys[i] = __fadd_rn(__fadd_rn(fabsf(y[i]), fabsf(__fmul_rn(k1[i], h))), ck::scal_min);   // >= 0.1
+      normal = normal && iys[i] < RCP_MAX;
     }
   }
+  if (normal) {
+#pragma unroll
+    for (int i = 0; i < NVM; i++)
+      if (i < NV) iys[i] = rcp_m(iys[i]);
+  } else {   // a state that has left the range of the FP32 step (infinities, NaN)
+#pragma unroll
+    for (int i = 0; i < NVM; i++)
+      if (i < NV) iys[i] = __fdiv_rn(1.0f, iys[i]);
+  }
+}
+
+// Largest of |a|, |b|, |c|, or NaN if one of them is.
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// The same of N values; three-input maxima, in two levels for the two-port models.
+template <int N>
+__device__ __forceinline__ float max_abs(const float *e) {
+  float m[(N + 2) / 3];
+#pragma unroll
+  for (int i = 0; i < N; i += 3) m[i / 3] = max3_abs(e[i], e[i + 1 < N ? i + 1 : i], e[i + 2 < N ? i + 2 : i]);
+  if constexpr (N <= 3) return m[0];
+  else return max_abs<(N + 2) / 3>(m);
 }
 
 // rk5_trial: one trial with h clamped to [hmin, hmax] (h keeps the clamped value): the
@@ -511,9 +537,11 @@ __device__ __forceinline__ float rk5_trial(const float *y, float &h, float hmin,
   const float f1 = __fmul_rn(h, ck::e1), f3 = __fmul_rn(h, ck::e3), f4 = __fmul_rn(h, ck::e4),
               f5 = __fmul_rn(h, ck::e5), f6 = __fmul_rn(h, ck::e6);
   // error terms two variables at a time (lane-exact, as in stage_comb)
-  float err = 0.0f;
+  float e[NVM];
 #pragma unroll
   for (int i = 0; i < NVM; i += (FIXED ? 2 : 1)) {
+    e[i] = 0.0f;
+    if (FIXED && i + 1 < NVM) e[i + 1] = 0.0f;
     if (i < NV) {
       if (FIXED && i + 1 < NVM) {
         float2 v = __fmul2_rn(make_float2(f1, f1), make_float2(k1[i], k1[i + 1]));
@@ -522,37 +550,60 @@ __device__ __forceinline__ float rk5_trial(const float *y, float &h, float hmin,
         v = __ffma2_rn(make_float2(f5, f5), make_float2(k5[i], k5[i + 1]), v);
         v = __ffma2_rn(make_float2(f6, f6), make_float2(k6[i], k6[i + 1]), v);
         v = __fmul2_rn(v, make_float2(iys[i], iys[i + 1]));
-        const float a0 = fabsf(v.x);
-        err = (err > a0) ? err : a0;
-        if (i + 1 < NV) {
-          const float a1 = fabsf(v.y);
-          err = (err > a1) ? err : a1;
-        }
+        e[i] = v.x;
+        if (i + 1 < NV) e[i + 1] = v.y;
       } else {
         float v = __fmaf_rn(f6, k6[i], __fmaf_rn(f5, k5[i], __fmaf_rn(f4, k4[i],
                                                                       __fmaf_rn(f3, k3[i], __fmul_rn(f1, k1[i])))));
-        float av = fabsf(__fmul_rn(v, iys[i]));
-        err = (err > av) ? err : av;
+        e[i] = __fmul_rn(v, iys[i]);
       }
     }
+  }
+  float err = 0.0f;
+  if constexpr (FIXED) {
+    err = max_abs<NVM>(e);
+    if (err != err) {     // the reference's scan forgets a NaN that a later variable follows
+      err = 0.0f;
+#pragma unroll
+      for (int i = 0; i < NVM; i++)
+        if (i < NV) err = (err > fabsf(e[i])) ? err : fabsf(e[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NVM; i++)
+      if (i < NV) err = (err > fabsf(e[i])) ? err : fabsf(e[i]);
   }
   return __fmul_rn(err, ck::inv_eps);
 }
 
 // Step size of the next trial after a rejection: max(0.9 h err^-1/4, 0.1 h).
 __device__ __forceinline__ float rk5_shrink(float h, float err) {
-  float hnew = __fmul_rn(__fmul_rn(h, ck::coeff), __fdiv_rn(1.0f, __fsqrt_rn(__fsqrt_rn(err))));
+  const float r4 = __fsqrt_rn(__fsqrt_rn(err));   // err > 1, or NaN
+  float hnew = __fmul_rn(__fmul_rn(h, ck::coeff), r4 < RCP_MAX ? rcp_m(r4) : __fdiv_rn(1.0f, r4));
   float h01 = __fmul_rn(0.1f, h);
   return (hnew > h01) ? hnew : h01;
 }
 
-// Step size proposed after an accepted trial: 0.9 h err^-1/5, or 5 h for a tiny error.
+// Step size proposed after an accepted trial: 0.9 h err^-1/5, or 5 h for a tiny error.  Both are
+// computed (no branch), so that the caller's next instructions overlap the chain of log and exp.
 __device__ __forceinline__ float rk5_grow(float h, float err, float hmin) {
-  if (err > ck::err_min) h = __fmul_rn(__fmul_rn(h, ck::coeff), exp_m(__fmul_rn(-0.2f, log_m(err))));
-  else h = __fmul_rn(5.0f, h);
-  if (!(h == h)) h = hmin;
-  return h;
+  const float hl = __fmul_rn(__fmul_rn(h, ck::coeff), exp_m(__fmul_rn(-0.2f, log_m(err))));
+  h = (err > ck::err_min) ? hl : __fmul_rn(5.0f, h);
+  return (h == h) ? h : hmin;
 }
+
+// The plain controller's step size between steps: the h and the error of the last accepted trial.
+// The growth is applied by the next step's beginning, where its chain (240 cycles) and that of the
+// first derivative run side by side, or before the state is stored.
+struct StepCtl {
+  float err = 0.0f;
+  bool grow = false;      // h is the last trial's and still to be grown
+  __device__ __forceinline__ void settle(float &h, float hmin) {
+    const float hg = rk5_grow(h, err, hmin);
+    h = grow ? hg : h;
+    grow = false;
+  }
+};
 
 // Largest step in [hmin, hmax] whose trial passes the error test (hmax if it passes, else a
 // bisection in log h with 30 halvings): the first trial a perfect proposal would choose.
@@ -587,7 +638,7 @@ __device__ __forceinline__ int rk5_step(double &x, float *y, float &h, float hmi
   float k1[NVM], yn[NVM], iys[NVM];
   rk5_begin(y, h, q, refr, k1, iys);
   if constexpr (LM == LM_BOUND) h = rk5_largest_passing(y, hmin, hmax, q, refr, k1, iys);
-  float f[(LM == LM_PLAIN || LM == LM_BOUND) ? 1 : SM_NF];
+  float f[LM == LM_BOUND ? 1 : SM_NF];
   if (LM == LM_LOG || (LM == LM_PROPOSE && h < hmax)) step_features<MODEL, PMAX>(y, k1, q.ports(), h, hmax, f);
   if (LM == LM_PROPOSE && h < hmax) {
     // the plain h would not reach the end of the time step: let the network propose
@@ -641,12 +692,36 @@ __device__ __forceinline__ bool aeif_external(const AeifArgs &A, const SpikeOut 
 template <int MODEL, int PMAX, bool FIXED, int LM>
 __device__ __forceinline__ bool aeif_substep(const AeifArgs &A, const SpikeOut &so, int i,
                                              const AeifQ<MODEL, PMAX, FIXED> &q, float *y, float &refr,
-                                             double &x, float &h, long long tidx, double tnow,
+                                             double &x, float &h, StepCtl &ctl, long long tidx, double tnow,
                                              unsigned long long &nd, const float *smodel, int &guard) {
   const double x1 = tnow;
   const float hmax = (float)(x1 - x);
-  nd += rk5_step<MODEL, PMAX, FIXED, LM>(x, y, h, A.hmin, A.hmin_acc, hmax, q, refr, so.status, smodel,
-                                         A.learn);
+  if constexpr (LM == LM_PLAIN) {
+    constexpr int NVM = 2 + AeifShape<MODEL>::npv * PMAX;
+    const int NV = 2 + AeifShape<MODEL>::npv * q.ports();
+    float k1[NVM], yn[NVM], iys[NVM];
+    ctl.settle(h, A.hmin);
+    rk5_begin(y, h, q, refr, k1, iys);
+    nd += 1;
+    for (int trials = 1;; trials++) {
+      ctl.err = rk5_trial(y, h, A.hmin, hmax, q, refr, k1, iys, yn);
+      nd += 5;
+      if (ctl.err <= 1.0f || h <= A.hmin_acc) break;
+      if (trials >= ck::max_trials) {
+        atomicOr(so.status, ST_RK5_TRIALS);
+        break;
+      }
+      h = rk5_shrink(h, ctl.err);
+    }
+    x += (double)h;
+    ctl.grow = true;
+#pragma unroll
+    for (int v = 0; v < NVM; v++)
+      if (v < NV) y[v] = yn[v];
+  } else {
+    nd += rk5_step<MODEL, PMAX, FIXED, LM>(x, y, h, A.hmin, A.hmin_acc, hmax, q, refr, so.status, smodel,
+                                           A.learn);
+  }
   return aeif_external(A, so, i, q, y, refr, x, tidx, tnow, guard);
 }
 
@@ -659,7 +734,10 @@ __device__ __forceinline__ bool aeif_external(const AeifArgs &A, const SpikeOut 
                                               double x, long long tidx, double tnow, int &guard) {
   const double x1 = tnow;
   const bool end = (x >= x1 - (double)A.hmin);
-  if (++guard > ck::max_substeps) {
+  ++guard;
+  const bool rare = guard > ck::max_substeps || y[0] < -1.0e3f || fabsf(y[1]) > 1.0e6f || refr > 0.0f || y[0] >= q.V_peak;
+  if (!rare) return end;
+  if (guard > ck::max_substeps) {
     atomicOr(so.status, ST_RK5_TRIALS);
     return true;
   }
@@ -767,11 +845,12 @@ __device__ __forceinline__ void warp_add(unsigned long long *ctr, unsigned long 
 template <int MODEL, int PMAX, bool FIXED>
 __device__ __forceinline__ bool aeif_tpi_iter(const AeifArgs &A, const SpikeOut &so, int i,
                                               const AeifQ<MODEL, PMAX, FIXED> &q, float *y, float &refr,
-                                              double &x, float &h, const StepT &t, float *k1, float *iys,
-                                              bool &open, int &trials, unsigned long long &nd, int &guard) {
+                                              double &x, float &h, StepCtl &ctl, const StepT &t, float *k1,
+                                              float *iys, bool &open, int &trials, unsigned long long &nd, int &guard) {
   constexpr int NVM = 2 + AeifShape<MODEL>::npv * PMAX;
   const int NV = 2 + AeifShape<MODEL>::npv * q.ports();
   if (!open) {
+    ctl.settle(h, A.hmin);
     rk5_begin(y, h, q, refr, k1, iys);
     nd += 1;
     trials = 0;
@@ -789,7 +868,8 @@ __device__ __forceinline__ bool aeif_tpi_iter(const AeifArgs &A, const SpikeOut 
   }
   open = false;
   x += (double)h;
-  h = rk5_grow(h, err, A.hmin);
+  ctl.err = err;
+  ctl.grow = true;
 #pragma unroll
   for (int v = 0; v < NVM; v++)
     if (v < NV) y[v] = yn[v];
@@ -842,6 +922,7 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
     // does not hold the others of its warp in that step; they go on with their next step.
     int m = 0, guard = 0;
     bool deferred = false;
+    StepCtl ctl;
     StepT t = step_at(cl, k0, 0, A.dt);
     double apf[PMAX];
     acc_prefetch<PMAX>(apf, q.ports(), A.n, i, A.in, 0);
@@ -856,7 +937,7 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
           break;
         }
         if (budget > 0) budget--;
-        if (aeif_tpi_iter(A, so, i, q, y, refr, x, h, t, k1, iys, open, trials, nd, guard)) {
+        if (aeif_tpi_iter(A, so, i, q, y, refr, x, h, ctl, t, k1, iys, open, trials, nd, guard)) {
           aeif_end_step(A, so, i, q, y, refr, m, t, rec_it0, apf, pc);
           guard = 0;
           if (++m < M) {
@@ -872,7 +953,7 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
           break;
         }
         if (budget > 0) budget--;
-        if (aeif_substep<MODEL, PMAX, FIXED, LM>(A, so, i, q, y, refr, x, h, t.tidx, t.tnow, nd, smodel,
+        if (aeif_substep<MODEL, PMAX, FIXED, LM>(A, so, i, q, y, refr, x, h, ctl, t.tidx, t.tnow, nd, smodel,
                                                  guard)) {
           aeif_end_step(A, so, i, q, y, refr, m, t, rec_it0, apf, pc);
           guard = 0;
@@ -883,6 +964,7 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
         }
       }
     }
+    if (LM == LM_PLAIN) ctl.settle(h, A.hmin);
     aeif_store<MODEL, PMAX, FIXED>(A, i, y, refr, x, h, NV);
     if (deferred) {
       const int pos = atomicAdd(A.strag_cnt, 1);
@@ -926,11 +1008,12 @@ __global__ void __launch_bounds__(128, 1) aeif_straggler_kernel(const AeifArgs A
     PoissonCache pc;
     poisson_cache_load(A.in, i, pc);
     int m = e.y, guard = 0;
+    StepCtl ctl;
     StepT t = step_at(cl, k0, m, A.dt);
     double apf[PMAX];
     acc_prefetch<PMAX>(apf, q.ports(), A.n, i, A.in, m);
     while (m < M) {
-      if (aeif_substep<MODEL, PMAX, FIXED, LM>(A, so, i, q, y, refr, x, h, t.tidx, t.tnow, nd, smodel, guard)) {
+      if (aeif_substep<MODEL, PMAX, FIXED, LM>(A, so, i, q, y, refr, x, h, ctl, t.tidx, t.tnow, nd, smodel, guard)) {
         aeif_end_step(A, so, i, q, y, refr, m, t, rec_it0, apf, pc);
         guard = 0;
         if (++m < M) {
@@ -939,6 +1022,7 @@ __global__ void __launch_bounds__(128, 1) aeif_straggler_kernel(const AeifArgs A
         }
       }
     }
+    if (LM == LM_PLAIN) ctl.settle(h, A.hmin);
     aeif_store<MODEL, PMAX, FIXED>(A, i, y, refr, x, h, NV);
   }
   warp_add(A.nderiv, nd);

@@ -899,6 +899,11 @@ int NGPU_GetLaunchMapping(int *vals, int n) {
   }, -1);
 }
 
+// Test hook: inputs on which the branch-free reciprocal and quotient differ from the compiler's.
+long long NGPU_TestRoundedOps() {
+  return guard([&] { return check_rounded_ops(); }, -1LL);
+}
+
 double NGPU_MeasureReductionRate(size_t bytes, long long n_ops) {
   return guard([&] { return measure_random_reduction_rate(bytes, n_ops); }, -1.0);
 }

@@ -476,6 +476,7 @@ void mark_sources_device(const std::vector<GenBlockDev> &blocks, const std::vect
 void set_launch_pdl(bool on);
 // reduction-rate probe (ngpu_probe.cu): 1e9 random FP64 reductions per second
 double measure_random_reduction_rate(size_t bytes, long long n_ops);
+long long check_rounded_ops();
 // STDP (ngpu_stdp.cu)
 int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);

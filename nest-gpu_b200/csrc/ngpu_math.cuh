@@ -20,6 +20,29 @@
 
 namespace ngpu {
 
+// Correctly rounded 1 / b for normal b below 2^126 without a branch, so that several pipeline (the
+// compiler's division and __frcp_rn each carry a branch to a slow path: the six of an RK5 step
+// were a serial chain of 430 of the step's 1900 cycles).  One Newton step with fused multiply-adds
+// from the hardware approximation: Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34 (1990), shows it correctly rounded from an
+// approximation within one ulp unless the significand of b is all ones, where the quotient lies
+// just above a power of two and the approximation is already the result.  The test compares it
+// with __frcp_rn over every float in range.
+__device__ __forceinline__ float rcp_m(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return __fmaf_rn(r, __fmaf_rn(-b, r, 1.0f), r);
+}
+constexpr float RCP_MAX = 8.507059173023462e37f;   // 2^126
+
+// Correctly rounded a / b for b in [1, 4) and |a| zero or in [2^-24, 1]: the same paper's division
+// step with the correctly rounded reciprocal; the remainder is exact in that range.
+__device__ __forceinline__ float div_m(float a, float b) {
+  const float r = rcp_m(b);
+  const float q = __fmul_rn(a, r);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+}
+
 // Both functions compute the main path for every input and select the special results
 // at the end (no branches).  rint(x log2 e) comes from the magic-number addition
 // 1.5 * 2^23, which rounds to the nearest integer, ties to even, like rintf for
@@ -45,9 +68,9 @@ __device__ __forceinline__ float exp_m(float x) {
   const int n2 = ni - n1;
   p = __fmul_rn(p, __uint_as_float((unsigned)(n1 + 127) << 23));
   p = __fmul_rn(p, __uint_as_float((unsigned)(n2 + 127) << 23));
-  p = (x > 88.72283935546875f) ? __int_as_float(0x7f800000) : p;
-  p = (x < -103.972084045410156f) ? 0.0f : p;
-  return (x == x) ? p : x;
+  // the special results are chosen beside the main path, which then ends in one select
+  const float sp = (x > 88.72283935546875f) ? __int_as_float(0x7f800000) : (x < -103.972084045410156f ? 0.0f : x);
+  return (x >= -103.972084045410156f && x <= 88.72283935546875f) ? p : sp;
 }
 
 __device__ __forceinline__ float log_m(float x) {
@@ -59,7 +82,7 @@ __device__ __forceinline__ float log_m(float x) {
   const bool hi = m > 1.41421354f;
   m = hi ? __fmul_rn(m, 0.5f) : m;
   e += hi ? 1 : 0;
-  const float s = __fdiv_rn(__fsub_rn(m, 1.0f), __fadd_rn(m, 1.0f));
+  const float s = div_m(__fsub_rn(m, 1.0f), __fadd_rn(m, 1.0f));   // m + 1 in [1.7, 2.42)
   const float s2 = __fmul_rn(s, s);
   float q = 9.09090936e-02f;
   q = __fmaf_rn(q, s2, 1.11111112e-01f);

@@ -7,6 +7,8 @@
 #include <stdexcept>
 #include <string>
 
+#include "ngpu_math.cuh"
+
 namespace ngpu {
 
 __global__ void random_reduction_kernel(double *buf, unsigned long long n_elem, long long ops_per_thread,
@@ -56,6 +58,36 @@ double measure_random_reduction_rate(size_t bytes, long long n_ops) {
   cudaFree(buf);
   probe_ok(err, "reduction probe");
   return (double)per * threads * blocks / (ms * 1e-3) / 1e9;
+}
+
+// ---------------------------------------------------------------------------
+// The branch-free reciprocal and quotient of ngpu_math.cuh against the compiler's correctly
+// rounded ones: every float from 1/16 up to 2^126, and every quotient that log_m forms.
+// ---------------------------------------------------------------------------
+__global__ void check_rounded_kernel(unsigned long long *bad) {
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  unsigned long long n = 0;
+  for (unsigned long long b = 0x3d800000ull + i0; b < 0x7e800000ull; b += stride) {
+    const float x = __uint_as_float((unsigned)b);
+    n += __float_as_uint(rcp_m(x)) != __float_as_uint(__frcp_rn(x));
+  }
+  for (unsigned long long b = 0x3f3504f0ull + i0; b <= 0x3fb504f8ull; b += stride) {   // sqrt(1/2) .. sqrt(2)
+    const float m = __uint_as_float((unsigned)b), num = __fsub_rn(m, 1.0f), den = __fadd_rn(m, 1.0f);
+    n += __float_as_uint(div_m(num, den)) != __float_as_uint(__fdiv_rn(num, den));
+  }
+  if (n) atomicAdd(bad, n);
+}
+
+// Number of inputs on which they differ (-1: the check could not run).
+long long check_rounded_ops() {
+  unsigned long long *d = nullptr, h = 0;
+  if (cudaMalloc(&d, sizeof(h)) != cudaSuccess) return -1;
+  cudaMemset(d, 0, sizeof(h));
+  check_rounded_kernel<<<148 * 8, 256>>>(d);
+  const bool ok = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess;
+  cudaFree(d);
+  return ok ? (long long)h : -1;
 }
 
 }  // namespace ngpu
