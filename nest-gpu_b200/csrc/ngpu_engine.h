@@ -89,6 +89,7 @@ struct Group {
   int gen0 = -1;                 // poiss_gen: first row in the generator table
   std::vector<uint32_t> pg_stream;   // poiss_gen: stream numbers (empty: index among generators)
   bool dirty = true;             // parameters changed since last upload
+  long long resident = 0;        // aeif: neurons resident at once in the uncapped update kernel
 };
 
 struct RecordSpec {
@@ -127,17 +128,19 @@ class Engine {
   int remote_spike_height = 0;
   float sim_time = 1000.0f;
   int graph_steps = 100;          // steps per captured CUDA graph
-  int rk5_budget = 4;             // RK5 steps per neuron before the straggler kernel takes over
+  int rk5_budget = -1;            // RK5 steps beyond the batch's length before the straggler kernel
+                                  // takes over (0: it never does; -1: by aeif_mapping)
   int deliver_blocks_req = 0;     // delivery grid size (0: from the number of spiking sources)
   int batch_max = MAX_BATCH;      // upper bound of the time-batch length (1: step by step)
-  int update_threads = 128;       // threads per block of the aeif update kernel (64, 128, 256)
+  int update_threads = 0;         // threads per block of the aeif update kernel (64, 128, 256; 0: 64)
   int deliver_group = 32;         // lanes per delivery work item (8, 16, 32)
   int deliver_aggregate = 0;      // 1: warp-aggregated reductions (with 32-lane work items)
   int deliver_prefetch = 0;       // 1: delivery loads the next work item's segment ahead
   int deliver_push = 0;           // 1: networks of iaf_psc_exp groups deliver each spike at emission
                                   // (set before calibration)
-  int update_occupancy = 0;       // 1: register-capped aeif update kernel
-  int update_trial_iter = 0;      // 1: aeif update kernel advances one RK5 trial per iteration
+  int update_occupancy = -1;      // 1, 2: register-capped aeif update kernel (-1: by aeif_mapping)
+  int update_trial_iter = -1;     // 1: aeif update kernel advances one RK5 trial per iteration (-1: by
+                                  // aeif_mapping)
   int persistent = -1;            // iaf-only networks: persistent cooperative step loop (-1: by persistent_auto)
   int launch_pdl = -1;            // programmatic dependent launch of the batch kernels (-1: one-step batches)
   int barrier_extra = 0;          // test hook: blocks the persistent loop's barriers wait for in excess
@@ -441,6 +444,7 @@ class Engine {
   SpikeOut spike_out() const;
   PushOut push_out() const;
   AeifArgs aeif_args(Group &g);
+  void aeif_mapping(const Group &g, AeifArgs &A) const;
   IafArgs iaf_args(Group &g);
   SpikeGenArgs sg_args(Group &g);
   ParrotArgs parrot_args(Group &g);
@@ -454,6 +458,7 @@ void engine_reset();
 // launchers (ngpu_kernels.cu)
 int launch_aeif(int model, const AeifArgs &A, const SpikeOut &so, const Clock *clk, int k0, int M,
                 cudaStream_t st);
+long long aeif_resident(int model, int nport, bool uniform);
 int launch_iaf(const IafArgs &A, const SpikeOut &so, const PushOut *po, const Clock *clk, int k0, int M,
                cudaStream_t st);
 int launch_iaf_multi(const IafArgs *tab, const int *blk0, int ngroups, int nblocks, const SpikeOut &so,

@@ -585,6 +585,36 @@ static int launch_aeif_m(const AeifArgs &A, const SpikeOut &so, const Clock *clk
   }
 }
 
+// Neurons of a model that are resident at once on the GPU in its update kernel without a register
+// cap (64-thread blocks).
+template <int MODEL, int PMAX, bool FIXED, bool UNI>
+static long long resident_k() {
+  int dev = 0, n_sm = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, aeif_batch_kernel<MODEL, PMAX, FIXED, LM_PLAIN, 0, UNI>, 64, 0);
+  return (long long)n_sm * per_sm * 64;
+}
+template <int MODEL>
+static long long resident_m(int nport, bool uniform) {
+  switch (nport) {
+  case 1: return uniform ? resident_k<MODEL, 1, true, true>() : resident_k<MODEL, 1, true, false>();
+  case 2: return uniform ? resident_k<MODEL, 2, true, true>() : resident_k<MODEL, 2, true, false>();
+  case 3: return uniform ? resident_k<MODEL, 3, true, true>() : resident_k<MODEL, 3, true, false>();
+  case 4: return uniform ? resident_k<MODEL, 4, true, true>() : resident_k<MODEL, 4, true, false>();
+  default: return resident_k<MODEL, MAX_PORT, false, false>();
+  }
+}
+long long aeif_resident(int model, int nport, bool uniform) {
+  switch (model) {
+  case M_AEIF_COND_BETA: return resident_m<M_AEIF_COND_BETA>(nport, uniform);
+  case M_AEIF_COND_ALPHA: return resident_m<M_AEIF_COND_ALPHA>(nport, uniform);
+  case M_AEIF_PSC_EXP: return resident_m<M_AEIF_PSC_EXP>(nport, uniform);
+  case M_AEIF_PSC_ALPHA: return resident_m<M_AEIF_PSC_ALPHA>(nport, uniform);
+  }
+  return 0;
+}
+
 int launch_aeif_learn(int model, const AeifArgs &A, const SpikeOut &so, const Clock *clk, int k0, int M,
                       cudaStream_t st);
 

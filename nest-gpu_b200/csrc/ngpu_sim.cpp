@@ -440,6 +440,11 @@ void Engine::calibrate() {
   d_clk_ = dalloc<Clock>(1);
   cuda_check(cudaMemset(d_clk_, 0, sizeof(Clock)), "clock");
   deliver_blocks_ = std::max(1, std::min(148 * 8, (n_src_out + 63) / 64));
+  // With slots of many megabytes fewer work items in flight keep fewer arrival steps open, so that
+  // the reductions stay in L2.  Blocks 296 / 592 / 1184, ms: 500k AdEx (8 MB a slot, 30 ms) 12.0 /
+  // 11.0 / 11.1, 1M (16 MB, 50 ms) 34.6 / 31.8 / 34.7, 2.8M ensemble (45 MB, 20 ms) 24.6 / 26.9 /
+  // 28.4; 250k and less take all the blocks there are.
+  while (deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184) deliver_blocks_ /= 2;
   if (plastic_) build_plastic(pl_edge, pl_key, pl_rank);
   // ---- dendritic delays: the reverse ring (plastic networks only; src/spike_buffer.cu:162-317)
   if (plastic_) {
@@ -629,6 +634,9 @@ void Engine::upload_params() {
         put(g, b + 2, t2);
         put(g, b + 3, pw);
       }
+      bool uniform = true;
+      for (float *p : g.d_der) uniform = uniform && !p;
+      g.resident = aeif_resident(g.model, g.nport, uniform);
     } else if (g.model == M_IAF_PSC_EXP) {
       g.der_val.assign(IP_NPAR, 0.0f);
       g.d_der.assign(IP_NPAR, nullptr);
@@ -796,6 +804,27 @@ PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
   return A;
 }
 
+// Launch mapping of a group's aeif update where the caller set none.
+// A group that is resident at once in the kernel without a register cap (aeif_resident: 66k
+// neurons for the two-port conductance model) loses nothing by letting a spiking neuron finish its
+// 40 to 60 sub-steps in its own warp; handing it to the straggler kernel would only add a launch to
+// the chain that sets the batch's length.  A larger group needs the block slots: neurons beyond a
+// step budget of M + 1 move to the straggler kernel, and the 96-register kernel with one trial per
+// iteration keeps the issue slots busy.  Measured, ms per 30 ms, 64-thread blocks, uncapped without
+// / capped with straggler kernel: 2-port beta 23k neurons 2.94 / 3.61, 40k 3.29 / 3.74, 60k 3.96 /
+// 3.96, 80k 5.71 / 4.19, 180k 9.35 / 5.58; 4-port 23k 3.23 / 3.97, 60k 5.77 / 4.47; psc_exp (per-
+// neuron parameters) 60k 2.88 / 3.68, 100k 3.58 / 4.00, 300k 7.75 / 6.45.  128-thread blocks are
+// the same or slower.  One-step batches pay the second launch every step: 80k 20.2 / 22.7, 180k
+// 25.4 / 25.7, so there the line lies at three waves.
+void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
+  const bool hand_off = A.hi - A.lo > (batch_ == 1 ? 3 * g.resident : g.resident);
+  const int budget = rk5_budget >= 0 ? rk5_budget : (hand_off ? 1 : 0);
+  A.budget = budget > 0 ? batch_ + budget : 0;
+  A.threads = update_threads > 0 ? update_threads : 64;
+  A.occupancy = update_occupancy >= 0 ? update_occupancy : (hand_off ? 2 : 0);
+  A.trial_iter = update_trial_iter >= 0 ? update_trial_iter : (hand_off ? 1 : 0);
+}
+
 AeifArgs Engine::aeif_args(Group &g) {
   AeifArgs A;
   std::memset(&A, 0, sizeof(A));
@@ -815,16 +844,13 @@ AeifArgs Engine::aeif_args(Group &g) {
   A.hmin = g.h_min_rel * dt;
   A.hmin_acc = A.hmin * 1.00001f;
   A.nderiv = d_counters_;
-  A.budget = rk5_budget > 0 ? batch_ + rk5_budget : 0;
   A.strag_list = g.d_strag;
   A.strag_cnt = d_strag_cnt_ + g.strag_slot;
   A.srec = spike_rec(g);
-  A.threads = update_threads;
-  A.occupancy = update_occupancy;
-  A.trial_iter = update_trial_iter;
   A.uniform = 1;
   for (int j = 0; j < AEIF_NSCAL + AEIF_NPORTPAR * g.nport && j < AEIF_NPAR; j++)
     if (g.d_der[j]) A.uniform = 0;
+  aeif_mapping(g, A);
   A.learn.mode = learn_mode_;
   A.learn.log = d_log_;
   A.learn.log_cursor = d_log_cursor_;
@@ -1583,6 +1609,12 @@ int Engine::autotune(int steps, std::vector<std::pair<std::string, double>> *log
   };
   if (persistent_eligible()) knobs.insert(knobs.begin(), single("persistent", &persistent, {0, 1}));
   if (deliver_blocks_req <= 0) deliver_blocks_req = base;
+  // the descent starts from explicit values where the mapping was automatic
+  if (update_threads <= 0) update_threads = 128;
+  if (update_occupancy < 0) update_occupancy = 0;
+  if (update_trial_iter < 0) update_trial_iter = 0;
+  if (rk5_budget < 0) rk5_budget = 4;
+  if (persistent < 0) persistent = persistent_auto(steps) ? 1 : 0;
   const float t = (float)steps * dt;
   auto trial = [&]() {
     invalidate_graphs();
