@@ -160,7 +160,7 @@ __global__ void moments_kernel(const float *feat, const float *target, long long
 // forward (inference) over a feature array
 // ---------------------------------------------------------------------------
 __global__ void mlp_forward_kernel(const float *model, const float *feat, int n, float *out) {
-  __shared__ float M[SM_NPAR];
+  __shared__ __align__(16) float M[SM_NPAR];
   for (int j = threadIdx.x; j < SM_NPAR; j += blockDim.x) M[j] = model[j];
   __syncthreads();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
