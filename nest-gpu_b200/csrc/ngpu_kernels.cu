@@ -472,7 +472,11 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
     float height;
     long long e0, e1;
   };
-  auto fetch = [&](int item) {
+  // (long segments are cut: the parts of a segment are consecutive work items)
+  const int lp = A.log2_parts;
+  const long long total_parts = (long long)total << lp;
+  auto fetch = [&](long long item_part) {
+    const int item = (int)(item_part >> lp), part = (int)(item_part & ((1 << lp) - 1));
     int lo = 0, hi = npairs;   // pair with s_pref[pr] <= item < s_pref[pr+1]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
@@ -490,6 +494,11 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
     it.height = __int_as_float(sp.y);
     it.e0 = __ldg(&A.ev_off[key]);
     it.e1 = __ldg(&A.ev_off[key + 1]);
+    if (lp) {
+      const long long c = (it.e1 - it.e0 + (1 << lp) - 1) >> lp;
+      it.e0 = min(it.e1, it.e0 + part * c);
+      it.e1 = min(it.e1, it.e0 + c);
+    }
     return it;
   };
   auto deliver = [&](const Item &it) {
@@ -521,9 +530,23 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
         if (valid && lane == __ffs(peers) - 1) atomicAdd(&acc[ew.x], v);
       }
     } else {
-      for (long long e = e0 + sub; e < e1; e += G) {
-        const uint2 ew = __ldg(reinterpret_cast<const uint2 *>(A.edge + e));
-        atomicAdd(&acc[ew.x], (double)__fmul_rn(height, __uint_as_float(ew.y)));
+      const uint2 *edge = reinterpret_cast<const uint2 *>(A.edge) + e0;
+      const int len = (int)(e1 - e0);
+      if (A.unroll) {          // four loads in flight per lane before their reductions
+        for (int e = sub; e < len; e += 4 * G) {
+          uint2 ew[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (e + u * G < len) ew[u] = __ldg(edge + e + u * G);
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (e + u * G < len) atomicAdd(&acc[ew[u].x], (double)__fmul_rn(height, __uint_as_float(ew[u].y)));
+        }
+      } else {
+        for (int e = sub; e < len; e += G) {
+          const uint2 ew = __ldg(edge + e);
+          atomicAdd(&acc[ew.x], (double)__fmul_rn(height, __uint_as_float(ew.y)));
+        }
       }
     }
     if (sub == 0) nev += (unsigned long long)(e1 - e0);
@@ -531,19 +554,19 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
   if constexpr (PF) {
     // software pipeline: the next item's ring entry and segment offsets are loaded before
     // this item's edges, so their dependent latencies overlap this item's traffic
-    int item = grp;
+    long long item = grp;
     Item cur;
-    if (item < total) cur = fetch(item);
-    while (item < total) {
-      const int next = item + ngrp;
+    if (item < total_parts) cur = fetch(item);
+    while (item < total_parts) {
+      const long long next = item + ngrp;
       Item nxt;
-      if (next < total) nxt = fetch(next);
+      if (next < total_parts) nxt = fetch(next);
       deliver(cur);
       cur = nxt;
       item = next;
     }
   } else {
-    for (int item = grp; item < total; item += ngrp) deliver(fetch(item));
+    for (long long item = grp; item < total_parts; item += ngrp) deliver(fetch(item));
   }
   // one counter update per block
   for (int o = 16; o > 0; o >>= 1) nev += __shfl_down_sync(0xffffffffu, nev, o);

@@ -445,6 +445,18 @@ void Engine::calibrate() {
   // 11.0 / 11.1, 1M (16 MB, 50 ms) 34.6 / 31.8 / 34.7, 2.8M ensemble (45 MB, 20 ms) 24.6 / 26.9 /
   // 28.4; 250k and less take all the blocks there are.
   while (deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184) deliver_blocks_ /= 2;
+  // Long (source, delay) segments are delivered in parts of about 128 edges (the four loads that a
+  // 32-lane group has in flight), so that a batch's few spikes fill the GPU: 12,500 neurons with
+  // 1250 edges per segment, 500 spikes a batch, 25.9 -> 12.3 us.  Networks with large accumulator
+  // slots have spikes enough, and more edges in flight only widen the set of addresses that L2 has
+  // to hold: parts and four loads per lane took 209 instead of 175 us on the 1M network (16 MB a
+  // slot) and 727 instead of 644 us on the 2.8M ensemble (45 MB).
+  deliver_unroll_ = (double)n_acc_ * sizeof(double) <= 12e6 ? 1 : 0;
+  deliver_log2_parts_ = 0;
+  if (n_src_out > 0 && deliver_unroll_) {
+    const double mean_len = (double)n_edge_dev_ / ((double)n_src_out * dspan_);
+    while (deliver_log2_parts_ < 4 && mean_len > (128 << deliver_log2_parts_)) deliver_log2_parts_++;
+  }
   if (plastic_) build_plastic(pl_edge, pl_key, pl_rank);
   // ---- dendritic delays: the reverse ring (plastic networks only; src/spike_buffer.cu:162-317)
   if (plastic_) {
@@ -936,6 +948,8 @@ DeliverArgs Engine::deliver_args() {
   A.n_pl = plastic_ ? stdp_.n_pl : 0;
   return A;
 }
+  A.log2_parts = deliver_log2_parts_;
+  A.unroll = deliver_unroll_;
 
 // ---------------------------------------------------------------------------
 // Plastic edges: forward index over the delivery CSR's (source, delay) segments, reverse

@@ -264,6 +264,8 @@ struct DeliverArgs {
   int *strag_cnt;        // per-group straggler counters, cleared for the batch
   int n_strag;
   int aggregate;         // 1 (with 32-lane groups): warp-aggregated reductions
+  int log2_parts;        // every segment is delivered in 2^log2_parts parts, a work group each
+  int unroll;            // 1: four edges in flight per lane
   int prefetch;          // 1: the next work item's ring entry and offsets loaded ahead
   int4 *xch;             // partitioned network: exchange buffer whose count the batch clears
   unsigned short *stamp; // plastic networks: arrival stamps [n_pl], reset at their wrap points
