@@ -923,9 +923,10 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
     for (int j = threadIdx.x; j < SM_NPAR; j += blockDim.x) smodel[j] = A.learn.model[j];
     __syncthreads();
   }
-  const int i = A.lo + blockIdx.x * blockDim.x + threadIdx.x;
+  // the first 2^log2_lanes lanes of every warp have a neuron
+  const int i = A.lo + (int)(((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << A.log2_lanes) + (int)(threadIdx.x & 31);
   unsigned long long nd = 0;
-  if (i < A.hi) {
+  if (i < A.hi && (threadIdx.x & 31) >> A.log2_lanes == 0) {
     AeifQ<MODEL, PMAX, FIXED> q;
     load_aeif_par<MODEL, PMAX, FIXED, UNI>(A, i, q);
     const int NV = 2 + S::npv * q.ports();
@@ -1054,7 +1055,8 @@ template <int MODEL, int PMAX, bool FIXED, int LM>
 int launch_aeif_p(const AeifArgs &A, const SpikeOut &so, const Clock *clk, int k0, int M, cudaStream_t st) {
   int tb = (A.threads == 64 || A.threads == 256) ? A.threads : 128;
   if (A.occupancy == 2 && tb > 128) tb = 128;   // the OCC = 2 variant is bounded to 128 threads
-  dim3 grid((A.hi - A.lo + tb - 1) / tb), block(tb);
+  const int per_block = (tb >> 5) << A.log2_lanes;
+  dim3 grid((A.hi - A.lo + per_block - 1) / per_block), block(tb);
   bool done = false;
   if constexpr (LM == LM_PLAIN && FIXED) {
     if (A.trial_iter && A.occupancy == 2 && A.uniform) {

@@ -835,6 +835,13 @@ void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
   A.threads = update_threads > 0 ? update_threads : 64;
   A.occupancy = update_occupancy >= 0 ? update_occupancy : (hand_off ? 2 : 0);
   A.trial_iter = update_trial_iter >= 0 ? update_trial_iter : (hand_off ? 1 : 0);
+  // The lanes of a warp wait for each other in every step (rejected trials, the network's
+  // proposals, a neighbour's spike), so a small group is spread thinner, over up to seven warps per
+  // SM.  Update kernel, us per batch, 32 neurons per warp / spread: 1000 neurons 75.4 / 66.6 (one
+  // per warp), with the step model 327 / 261; but 23k neurons 81 / 88.6 at 16 per warp (ten warps
+  // per SM) and 6000 55.9 / 56.5 at four: more warps than that slow each other down.
+  A.log2_lanes = 5;
+  while (A.log2_lanes > 0 && (A.hi - A.lo) <= (148LL * 7 << (A.log2_lanes - 1))) A.log2_lanes--;
 }
 
 AeifArgs Engine::aeif_args(Group &g) {

@@ -176,6 +176,7 @@ struct AeifArgs {
   unsigned long long *nderiv;
   int budget;            // RK5 steps per neuron and batch in the main kernel (0: no limit)
   int threads;           // threads per block of the main kernel (64, 128 or 256)
+  int log2_lanes;        // neurons per warp of the main kernel: 2^log2_lanes
   int occupancy;         // 1: register-capped variant of the main kernel (more resident warps)
   int uniform;           // 1: every parameter is uniform over the group (no parameter arrays)
   int trial_iter;        // 1: main kernel advances one RK5 trial per loop iteration
@@ -263,9 +264,9 @@ struct DeliverArgs {
   unsigned long long *n_events;
   int *strag_cnt;        // per-group straggler counters, cleared for the batch
   int n_strag;
-  int aggregate;         // 1 (with 32-lane groups): warp-aggregated reductions
   int log2_parts;        // every segment is delivered in 2^log2_parts parts, a work group each
   int unroll;            // 1: four edges in flight per lane
+  int aggregate;         // 1 (with 32-lane groups): warp-aggregated reductions
   int prefetch;          // 1: the next work item's ring entry and offsets loaded ahead
   int4 *xch;             // partitioned network: exchange buffer whose count the batch clears
   unsigned short *stamp; // plastic networks: arrival stamps [n_pl], reset at their wrap points
