@@ -83,10 +83,14 @@ __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so,
   const long long rec_it0 = cl.rec_it0;
   PoissonCache pc;
   poisson_cache_load(A.in, i, pc);
+  // the input of the step after next is on its way while a step is integrated
+  double apf[2], next[2];
+  acc_prefetch<2>(apf, 2, n, i, A.in, 0);
+  acc_prefetch<2>(next, M > 1 ? 2 : 0, n, i, A.in, 1);
   for (int m = 0; m < M; m++) {
     const StepT t = step_at(cl, k0, m, A.dt);
-    double apf[2];
-    acc_prefetch<2>(apf, 2, n, i, A.in, m);
+    double after[2];
+    acc_prefetch<2>(after, m + 2 < M ? 2 : 0, n, i, A.in, m + 2);
     if (iaf_step(q)) push_spike(so, A.srec, A.i0 + i, i, 1.0f, t.tidx, t.tnow);
     if (A.rec.first) {
       const float yr[4] = {q.Iex, q.Iin, q.V, q.refr};
@@ -95,6 +99,10 @@ __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so,
     double in[2];
     step_inputs_pf<2>(in, apf, 2, n, i, A.in, pc, m, t.tidx, t.tnow);
     iaf_fold(q, in);
+    apf[0] = next[0];
+    apf[1] = next[1];
+    next[0] = after[0];
+    next[1] = after[1];
   }
   iaf_store(A, i, q);
 }
@@ -657,9 +665,16 @@ int launch_aeif(int model, const AeifArgs &A, const SpikeOut &so, const Clock *c
 int launch_iaf(const IafArgs &A, const SpikeOut &so, const PushOut *po, const Clock *clk, int k0, int M,
                cudaStream_t st) {
   if (A.hi <= A.lo) return 0;
-  const dim3 g((A.hi - A.lo + 255) / 256), b(256);
-  if (po) launch_k(iaf_push_batch_kernel, g, b, 0, st, A, so, *po, clk, k0, M);
-  else launch_k(iaf_batch_kernel, g, b, 0, st, A, so, clk, k0, M);
+  const int n = A.hi - A.lo;
+  const dim3 g((n + 255) / 256), b(256);
+  if (po) {
+    launch_k(iaf_push_batch_kernel, g, b, 0, st, A, so, *po, clk, k0, M);
+  } else {
+    // small groups in 64-thread blocks, so that they reach every SM (12,500 neurons:
+    // 18.5 -> 18.0 us per 15-step batch)
+    const int tb = n < 148 * 256 ? 64 : 256;
+    launch_k(iaf_batch_kernel, dim3((n + tb - 1) / tb), dim3(tb), 0, st, A, so, clk, k0, M);
+  }
   return 1;
 }
 
