@@ -948,6 +948,8 @@ DeliverArgs Engine::deliver_args() {
   A.n_events = d_counters_ + 1;
   A.strag_cnt = d_strag_cnt_;
   A.n_strag = n_strag_;
+  A.log2_parts = deliver_log2_parts_;
+  A.unroll = deliver_unroll_;
   A.aggregate = deliver_aggregate;
   A.prefetch = deliver_prefetch;
   A.xch = part_world_ > 1 ? xch_send_ : nullptr;
@@ -955,8 +957,6 @@ DeliverArgs Engine::deliver_args() {
   A.n_pl = plastic_ ? stdp_.n_pl : 0;
   return A;
 }
-  A.log2_parts = deliver_log2_parts_;
-  A.unroll = deliver_unroll_;
 
 // ---------------------------------------------------------------------------
 // Plastic edges: forward index over the delivery CSR's (source, delay) segments, reverse
@@ -1472,8 +1472,6 @@ void Engine::simulation_step() {
   run_steps(1);
   it_ += 1;
   cuda_check(cudaStreamSynchronize(stream_), "step");
-  Clock c;
-  cuda_check(cudaMemcpy(&c, d_clk_, sizeof(Clock), cudaMemcpyDeviceToHost), "clock");
   neural_time_ = neur_t0_ + (double)dt * (double)it_;
 }
 
