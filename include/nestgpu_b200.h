@@ -297,8 +297,8 @@ int NGPU_SetDeliverBlocks(int n);
 int NGPU_SetBatchMax(int n);
 
 /* RK5 steps a neuron may take in the main update kernel per batch beyond one per time step
-   before it is handed to the straggler kernel (default 4; 0 = no hand-off).  Results do not
-   depend on it. */
+   before it is handed to the straggler kernel (0 = no hand-off; without a call chosen from the
+   network's size).  Results do not depend on it. */
 int NGPU_SetRk5Budget(int n);
 
 /* Pack a device-resident edge list into the spike-delivery layout: edges grouped into
@@ -337,7 +337,7 @@ int NGPU_SetGraphSteps(int n);
    launch (the minimum delay in steps + 1, at most 32 and at most the batch_max setting). */
 int NGPU_GetBatchLength(void);
 
-/* Threads per block of the aeif update kernel (64, 128 or 256; default 128). */
+/* Threads per block of the aeif update kernel (64, 128 or 256; without a call 64). */
 int NGPU_SetUpdateThreads(int n);
 /* 1: use the register-capped variant of the aeif update kernel (three 256-thread blocks per
    SM, more warps in flight, a few register spills); 2: with the trial-per-iteration update
@@ -371,10 +371,10 @@ int NGPU_DeliverPushActive(void);
    segment of one (source, delay) pair; short segments leave fewer lanes idle with small
    groups. */
 int NGPU_SetDeliverGroup(int g);
-/* 1: a network whose neurons are all iaf_psc_exp runs its steps in one cooperative launch per
-   CUDA-graph's worth of steps (delivery and update separated by grid barriers with bounded
-   waits); 0 (default): per-batch launches in CUDA graphs.  Results are the same either way; the
-   autotuner tries both. */
+/* 1: a network whose neurons are all iaf_psc_exp (and that fits one neuron per thread) runs its
+   steps in cooperative launches with one grid barrier with a bounded wait per step; 0: per-batch
+   launches in CUDA graphs.  Without a call the engine chooses: the cooperative loop for minimum
+   delays of one step.  Results are the same either way; the autotuner tries both. */
 int NGPU_SetPersistent(int on);
 /* 1: the kernels of a time batch are launched with programmatic stream serialization, so each
    kernel's launch and block scheduling overlap the end of the kernel before it (every such

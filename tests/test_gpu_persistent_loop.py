@@ -45,7 +45,7 @@ def _state(api, pops):
 
 
 @pytest.mark.parametrize("n,lo,hi", [(2, 0.1, 0.1), (147, 0.1, 0.2), (149, 0.1, 3.0), (1000, 0.2, 0.2), (1000, 0.2, 1.7),
-                                     (700, 0.3, 2.0), (300, 1.5, 1.5), (900, 0.1, 25.6)])
+                                     (700, 0.3, 2.0), (300, 1.5, 1.5), (900, 0.1, 19.2)])
 def test_delay_ranges_match_oracle(n, lo, hi):
     ngpu.SetPersistent(True)
     pops = _net(ngpu, n, lo, hi)
@@ -61,7 +61,7 @@ def test_delay_ranges_match_oracle(n, lo, hi):
     assert ngpu.GetStats()["n_events"] == o.NEvents() and ngpu.GetStats()["status"] == 0
 
 
-@pytest.mark.parametrize("n,hi", [(576 * 148, 1.0), (576 * 148 + 1, 1.0), (400, 25.7)])
+@pytest.mark.parametrize("n,hi", [(576 * 148, 1.0), (576 * 148 + 1, 1.0), (400, 19.3)])
 def test_capacity_and_what_lies_beyond_it(n, hi):
     """The largest network of the loop, one neuron more, and one delay group too many (the last
     two run in the per-batch kernels) equal the per-batch kernels."""
