@@ -417,7 +417,7 @@ class Engine {
   int pers_blocks_ = 0;          // blocks of the persistent loop (0: it cannot run this network)
   bool push_eligible() const;
   bool iaf_only() const;
-  void run_persistent(int steps);
+  bool run_persistent(int steps);
 
   template <class T> T *dalloc(size_t n);
   void free_device();

@@ -1206,15 +1206,22 @@ bool Engine::iaf_only() const {
   return any;
 }
 
-// `steps` steps in one cooperative launch of the persistent loop, then the clock advance.
-void Engine::run_persistent(int steps) {
+// `steps` steps in one cooperative launch of the persistent loop, then the clock advance; false if
+// the launch was refused and the loop was the engine's own choice (the caller goes on per batch).
+bool Engine::run_persistent(int steps) {
   cuda_check(cudaMemsetAsync(d_bar_, 0, sizeof(GridBarrier), stream_), "barrier reset");
   const int r = launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_,
                                       steps, d_bar_, kernel_seed, pers_blocks_, barrier_extra, stream_);
+  if (r < 0 && persistent < 0) {
+    cudaGetLastError();
+    persistent = 0;
+    return false;
+  }
   if (r < 0) throw NgpuError(std::string("cooperative launch of the persistent step loop failed: ") +
                              cudaGetErrorString(cudaGetLastError()));
   launch_clock_advance(d_clk_, steps, stream_);
   n_launch_ += 2;
+  return true;
 }
 
 void Engine::ensure_record_window(long long rows) {
@@ -1289,7 +1296,7 @@ void Engine::run_steps(long long n) {
     window = std::min<long long>(n, REC_WINDOW);
     ensure_record_window(window);
   }
-  const bool pers = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(n));
+  bool pers = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(n));
   if (pers) prepare_multi();
   long long done = 0;
   while (done < n) {
@@ -1298,8 +1305,8 @@ void Engine::run_steps(long long n) {
     while (left > 0) {
       if (pers) {
         const int steps = (int)std::min<long long>(PERS_STEPS, left);
-        run_persistent(steps);
-        left -= steps;
+        pers = run_persistent(steps);
+        if (pers) left -= steps;
         continue;
       }
       const int steps = (int)std::min<long long>(K, left);
