@@ -424,6 +424,11 @@ __device__ __forceinline__ void reset_stamps(const DeliverArgs &A, long long T, 
   }
 }
 
+// One edge (accumulator index, weight) on its way to the accumulators.  Read through L2: with
+// programmatic launch this kernel is already resident while the previous step's plasticity kernels
+// write weights, and the read-only path asks for data that no one writes during the kernel's life.
+__device__ __forceinline__ uint2 load_edge(const EdgeW *e) { return __ldcg(reinterpret_cast<const uint2 *>(e)); }
+
 // The delivery of one batch by block `block` of `nblocks`; s_pref holds dspan*M+1 ints.
 template <int G, bool AGG = false, bool PF = false>
 __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock *clk, int k0, int M, int *s_pref,
@@ -493,8 +498,7 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
     const int m = lo / A.dspan, dd = lo - m * A.dspan;
     const int j = item - s_pref[lo];
     const long long te = t_first + m - 1 - (A.dmin + dd);
-    // segment offsets and edges are written by no kernel that delivers (the persistent loop
-    // writes ring entries between its deliveries): read-only path for those two
+    // the segment offsets are written at calibration only: read-only path
     const int2 sp = A.ring[(size_t)(te % A.R) * A.cap + j];
     const size_t key = (size_t)sp.x * A.dspan + dd;
     Item it;
@@ -524,7 +528,7 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
         const long long e = base + lane;
         const bool valid = e < e1;
         uint2 ew = make_uint2(0xffffffffu, 0u);
-        if (valid) ew = __ldg(reinterpret_cast<const uint2 *>(A.edge + e));
+        if (valid) ew = load_edge(A.edge + e);
         double v = valid ? (double)__fmul_rn(height, __uint_as_float(ew.y)) : 0.0;
         const unsigned peers = __match_any_sync(0xffffffffu, ew.x);
         if (__any_sync(0xffffffffu, __popc(peers) > 1)) {
@@ -538,21 +542,21 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
         if (valid && lane == __ffs(peers) - 1) atomicAdd(&acc[ew.x], v);
       }
     } else {
-      const uint2 *edge = reinterpret_cast<const uint2 *>(A.edge) + e0;
+      const EdgeW *edge = A.edge + e0;
       const int len = (int)(e1 - e0);
       if (A.unroll) {          // four loads in flight per lane before their reductions
         for (int e = sub; e < len; e += 4 * G) {
           uint2 ew[4];
 #pragma unroll
           for (int u = 0; u < 4; u++)
-            if (e + u * G < len) ew[u] = __ldg(edge + e + u * G);
+            if (e + u * G < len) ew[u] = load_edge(edge + e + u * G);
 #pragma unroll
           for (int u = 0; u < 4; u++)
             if (e + u * G < len) atomicAdd(&acc[ew[u].x], (double)__fmul_rn(height, __uint_as_float(ew[u].y)));
         }
       } else {
         for (int e = sub; e < len; e += G) {
-          const uint2 ew = __ldg(edge + e);
+          const uint2 ew = load_edge(edge + e);
           atomicAdd(&acc[ew.x], (double)__fmul_rn(height, __uint_as_float(ew.y)));
         }
       }
