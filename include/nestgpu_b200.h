@@ -384,6 +384,9 @@ int NGPU_SetPersistent(int on);
    (default) uses it for batches of one time step only (a minimum delay of one step), where a
    step is two short launches.  The autotuner tries both.  No counterpart in the reference. */
 int NGPU_SetProgrammaticLaunch(int on);
+/* Test hook: sets the calling thread's programmatic-launch switch (on < 0: leaves it) and returns
+   it; the engine sets it around the launches of a time batch. */
+int NGPU_TestLaunchSwitch(int on);
 /* Test hook: number of inputs on which the engine's branch-free reciprocal and quotient differ
    from the correctly rounded ones (0), over the whole range in which they are used. */
 long long NGPU_TestRoundedOps();

@@ -50,8 +50,9 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Set by the engine around the launches of one time batch (ngpu_kernels.cu).
-extern bool g_launch_pdl;
+// Set by the engine around the launches of one time batch (ngpu_kernels.cu), for the calling
+// thread: each host thread has an engine of its own.
+extern thread_local bool g_launch_pdl;
 
 // kern<<<grid, block, smem, st>>>(args...), with programmatic stream serialization when
 // g_launch_pdl is set.

@@ -899,6 +899,15 @@ int NGPU_GetLaunchMapping(int *vals, int n) {
   }, -1);
 }
 
+// Test hook: sets the calling thread's programmatic-launch switch (on < 0: leaves it) and
+// returns it.
+int NGPU_TestLaunchSwitch(int on) {
+  return guard([&] {
+    if (on >= 0) set_launch_pdl(on != 0);
+    return get_launch_pdl() ? 1 : 0;
+  }, -1);
+}
+
 // Test hook: inputs on which the branch-free reciprocal and quotient differ from the compiler's.
 long long NGPU_TestRoundedOps() {
   return guard([&] { return check_rounded_ops(); }, -1LL);

@@ -481,6 +481,7 @@ int launch_exchange_unpack(const SpikeOut &so, const int4 *recv, int xch_cap, in
 void mark_sources_device(const std::vector<GenBlockDev> &blocks, const std::vector<RuleBlockDev> &rblocks,
                          unsigned char *d_flag, cudaStream_t st);
 void set_launch_pdl(bool on);
+bool get_launch_pdl();
 // reduction-rate probe (ngpu_probe.cu): 1e9 random FP64 reductions per second
 double measure_random_reduction_rate(size_t bytes, long long n_ops);
 long long check_rounded_ops();

@@ -24,8 +24,9 @@
 
 namespace ngpu {
 
-bool g_launch_pdl = false;
+thread_local bool g_launch_pdl = false;
 void set_launch_pdl(bool on) { g_launch_pdl = on; }
+bool get_launch_pdl() { return g_launch_pdl; }
 
 // Delivery at emission: the block adds the out-edges of node `src`, which spiked at time
 // index `tidx`, into the accumulator ring.  The source's edges are contiguous in the CSR,

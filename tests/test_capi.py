@@ -232,3 +232,17 @@ def test_syn_group_status_like_reference_log():
     assert ngpu.GetStatus(g, ["fact", "offset"]) == [5.0, 6.0]
     assert ngpu.GetStatus(g, ["offset", "fact"]) == [6.0, 5.0]
     ngpu.Reset()
+
+
+def test_programmatic_launch_switch_is_per_thread():
+    """Each host thread has an engine of its own; one engine's launches must not turn another's
+    into programmatic ones in the middle of a batch."""
+    import threading
+    sw = ngpu._lib.NGPU_TestLaunchSwitch
+    seen = []
+    assert sw(1) == 1
+    t = threading.Thread(target=lambda: seen.extend([sw(-1), sw(0)]))
+    t.start()
+    t.join()
+    assert seen == [0, 0] and sw(-1) == 1
+    assert sw(0) == 0
