@@ -411,10 +411,11 @@ int NGPU_TestTensorWaitTimeout(int on);
    values. */
 int NGPU_Autotune(int steps, int *update_threads, int *deliver_group, int *deliver_blocks,
                   int *rk5_budget);
-/* The current launch mapping: writes min(n, 10) of {update block size, register-capped update
-   variant, delivery lane group, delivery grid (0: automatic), RK5 step budget, persistent loop,
-   programmatic launch, trial-per-iteration update, warp-aggregated delivery, pipelined delivery}
-   and returns 10 (-1 on error).  No counterpart in the reference. */
+/* The launch mapping in use: writes min(n, 10) of {update block size, register-capped update
+   variant, delivery lane group, delivery grid (0: automatic), RK5 step budget, persistent loop
+   (1: long calls run in it), programmatic launch (-1: automatic), trial-per-iteration update,
+   warp-aggregated delivery, pipelined delivery} and returns 10 (-1 on error).  What no call has
+   set is reported as the engine chooses it, for the largest aeif group where groups differ.  No counterpart in the reference. */
 int NGPU_GetLaunchMapping(int *vals, int n);
 /* Measured rate (1e9 per second) of FP64 reductions to uniformly random addresses of a
    `bytes`-byte device buffer, `n_ops` in total: the access pattern of the spike delivery's

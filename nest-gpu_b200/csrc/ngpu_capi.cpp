@@ -881,19 +881,20 @@ int NGPU_SetProgrammaticLaunch(int on) {
 int NGPU_Autotune(int steps, int *update_threads, int *deliver_group, int *deliver_blocks, int *rk5_budget) {
   return guard([&] {
     const int n = E().autotune(steps, nullptr);
-    if (update_threads) *update_threads = E().update_threads;
+    const Engine::Mapping m = E().mapping_in_use();
+    if (update_threads) *update_threads = m.threads;
     if (deliver_group) *deliver_group = E().deliver_group;
     if (deliver_blocks) *deliver_blocks = E().deliver_blocks_req;
-    if (rk5_budget) *rk5_budget = E().rk5_budget;
+    if (rk5_budget) *rk5_budget = m.budget;
     return n;
   }, -1);
 }
 
 int NGPU_GetLaunchMapping(int *vals, int n) {
   return guard([&] {
-    const int v[10] = {E().update_threads, E().update_occupancy, E().deliver_group, E().deliver_blocks_req,
-                       E().rk5_budget, E().persistent, E().launch_pdl, E().update_trial_iter,
-                       E().deliver_aggregate, E().deliver_prefetch};
+    const Engine::Mapping m = E().mapping_in_use();
+    const int v[10] = {m.threads, m.occupancy, E().deliver_group, E().deliver_blocks_req, m.budget, m.persistent,
+                       E().launch_pdl, m.trial_iter, E().deliver_aggregate, E().deliver_prefetch};
     for (int i = 0; i < n && i < 10; i++) vals[i] = v[i];
     return 10;
   }, -1);

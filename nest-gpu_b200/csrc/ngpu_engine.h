@@ -273,6 +273,13 @@ class Engine {
   void step_bound_mode(bool on);
   int learn_mode() const { return learn_mode_; }
   int batch_length() const { return batch_; }
+  // The launch mapping in use: what is automatic as it is resolved, for the largest aeif group
+  // (as for a small one before calibration).
+  struct Mapping {
+    int threads, occupancy, trial_iter, budget;   // aeif update
+    int persistent;                               // 1: long calls run in the persistent loop
+  };
+  Mapping mapping_in_use() const;
   // captured graphs hold the launch mappings: drop them when a mapping knob changes
   void invalidate_graphs();
 

@@ -844,6 +844,22 @@ void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
   while (A.log2_lanes > 0 && (A.hi - A.lo) <= (148LL * 7 << (A.log2_lanes - 1))) A.log2_lanes--;
 }
 
+Engine::Mapping Engine::mapping_in_use() const {
+  const Group none;
+  const Group *big = &none;
+  for (auto &g : groups_)
+    if (is_aeif(g.model) && g.hi - g.lo > big->hi - big->lo) big = &g;
+  AeifArgs A;
+  std::memset(&A, 0, sizeof(A));
+  A.lo = big->lo;
+  A.hi = big->hi;
+  aeif_mapping(*big, A);
+  Mapping m{A.threads, A.occupancy, A.trial_iter, A.budget > 0 ? A.budget - batch_ : 0, 0};
+  if (!calibrated_) m.persistent = persistent > 0;
+  else m.persistent = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(1LL << 30));
+  return m;
+}
+
 AeifArgs Engine::aeif_args(Group &g) {
   AeifArgs A;
   std::memset(&A, 0, sizeof(A));

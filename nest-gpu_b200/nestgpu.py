@@ -1564,8 +1564,10 @@ def MeasureReductionRate(nbytes, n_ops):
 
 
 def GetLaunchMapping():
-    """The current launch mapping (engine extension): update block size and variant, delivery
-    lane group and grid, RK5 step budget, persistent loop and programmatic launch."""
+    """The launch mapping in use (engine extension): update block size and variant, delivery
+    lane group and grid (0: automatic), RK5 step budget, persistent loop (1: long calls run in it)
+    and programmatic launch (-1: automatic).  What no call has set is given as the engine chooses
+    it, for the largest aeif group where groups differ."""
     _need_b200("GetLaunchMapping")
     v = (ctypes.c_int * 10)()
     _c["NGPU_GetLaunchMapping"](v, 10)

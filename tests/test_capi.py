@@ -246,3 +246,17 @@ def test_programmatic_launch_switch_is_per_thread():
     t.join()
     assert seen == [0, 0] and sw(-1) == 1
     assert sw(0) == 0
+
+
+def test_launch_mapping_reports_what_is_in_use():
+    """What no call has set is reported as the engine would choose it, not as a placeholder; what a
+    call has set is reported as set."""
+    m = ngpu.GetLaunchMapping()
+    assert m["update_threads"] in (64, 128, 256) and m["update_occupancy"] in (0, 1, 2)
+    assert m["rk5_budget"] >= 0 and m["update_trial_iter"] in (0, 1) and m["persistent"] in (0, 1)
+    ngpu.SetUpdateThreads(256)
+    ngpu.SetRk5Budget(3)
+    ngpu.SetUpdateOccupancy(2)
+    ngpu.SetPersistent(True)
+    m = ngpu.GetLaunchMapping()
+    assert (m["update_threads"], m["rk5_budget"], m["update_occupancy"], m["persistent"]) == (256, 3, 2, 1)

@@ -1,0 +1,51 @@
+"""The launch mapping that the engine chooses where no call sets one: what GetLaunchMapping reports
+of it, and how Autotune starts from it and leaves it."""
+import pytest
+
+import nestgpu as ngpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def fresh_engine():
+    ngpu.Reset()
+    ngpu.SetVerbosityLevel(0)
+    yield
+    ngpu.Reset()
+
+
+def _aeif(n):
+    neuron = ngpu.Create("aeif_cond_beta_multisynapse", n, 2)
+    ngpu.SetStatus(neuron, {"E_rev": [0.0, -85.0], "I_e": 600.0})
+    ngpu.ConnectFixedIndegreeGPU(neuron, neuron, 2, 0.1, 1.0, 1.5, receptor=0, seed=1)
+    return neuron
+
+
+def _iaf(n, lo=0.1, hi=0.5):
+    neuron = ngpu.Create("iaf_psc_exp", n)
+    ngpu.SetStatus(neuron, "I_e", 600.0)
+    ngpu.ConnectFixedIndegreeGPU(neuron, neuron, 3, 1.0, lo, hi, receptor=0, seed=1)
+    return neuron
+
+
+# 64-thread blocks; beyond the neurons resident at once the hand-off and the capped kernel
+@pytest.mark.parametrize("n,want", [(2000, (64, 0, 0, 0)), (150000, (64, 2, 1, 1))])
+def test_automatic_aeif_mapping_is_reported(n, want):
+    _aeif(n)
+    ngpu.Simulate(1.0)
+    m = ngpu.GetLaunchMapping()
+    assert (m["update_threads"], m["update_occupancy"], m["update_trial_iter"], m["rk5_budget"]) == want
+
+
+@pytest.mark.parametrize("n,lo,hi,forced,want", [(500, 0.1, 0.5, None, 1), (500, 1.0, 1.5, None, 0), (500, 1.0, 1.5, True, 1),
+                                                 (500, 0.1, 0.5, False, 0), (500, 0.1, 19.3, True, 0)])
+def test_persistent_loop_in_use_is_reported(n, lo, hi, forced, want):
+    _iaf(n, lo, hi)
+    if forced is not None:
+        ngpu.SetPersistent(forced)
+    ngpu.Simulate(2.0)
+    assert ngpu.GetLaunchMapping()["persistent"] == want
+    l0 = ngpu.GetLaunchCount()
+    ngpu.Simulate(2.0)
+    assert (ngpu.GetLaunchCount() - l0 == 2) == bool(want)
