@@ -396,6 +396,11 @@ long long NGPU_TestRoundedOps();
    (a second or two); the kernel records the timeout and returns, and the Simulate call fails
    with error code 2 while the GPU context stays usable.  0 (default) disables it. */
 int NGPU_TestBarrierTimeout(int extra);
+/* Test hook for the start of the persistent loop: with how = 1 its cooperative launch counts as
+   refused; with how = 2 its blocks wait at the start for one block more than the launch has, give
+   up after some 20 ms and leave the state as it is, and the engine runs the steps in per-batch
+   launches.  0 (default) disables it. */
+int NGPU_TestLoopStart(int how);
 /* Test hook for the failure path of the step-model training kernel: with on != 0 its
    tensor-core products are issued but their completion is never signalled on the block's
    mbarrier, so the bounded wait runs out; the kernel records it, releases its tensor memory

@@ -853,6 +853,15 @@ int NGPU_TestBarrierTimeout(int extra) {
   }, -1);
 }
 
+// Test hook of the persistent loop's start: 1: its launch counts as refused; 2: its gate waits for
+// one block more than the launch has and closes; 0: off.
+int NGPU_TestLoopStart(int how) {
+  return guard([&] {
+    E().loop_start_test = how == 1 || how == 2 ? how : 0;
+    return 0;
+  }, -1);
+}
+
 // Test hook: the training kernel's tensor-core products complete unsignalled, so its bounded
 // wait runs out and the call fails.
 int NGPU_TestTensorWaitTimeout(int on) {
@@ -864,8 +873,7 @@ int NGPU_TestTensorWaitTimeout(int on) {
 
 int NGPU_SetPersistent(int on) {
   return guard([&] {
-    E().persistent = on ? 1 : 0;
-    E().invalidate_graphs();
+    E().set_persistent(on ? 1 : 0);
     return 0;
   }, -1);
 }

@@ -143,6 +143,8 @@ class Engine {
                                   // aeif_mapping)
   int persistent = -1;            // iaf-only networks: persistent cooperative step loop (-1: by persistent_auto)
   int launch_pdl = -1;            // programmatic dependent launch of the batch kernels (-1: one-step batches)
+  int loop_start_test = 0;        // test hook: 1: the persistent loop's launch counts as refused, 2: its gate
+                                  // waits for one block more than the launch has
   int barrier_extra = 0;          // test hook: blocks the persistent loop's barriers wait for in excess
   bool use_device_rng = true;     // cuRAND device generator (as the reference) if a GPU exists
 
@@ -417,6 +419,8 @@ class Engine {
   int *d_iaf_blk0_ = nullptr;
   int *d_iaf_first_ = nullptr;   // neuron prefix over the iaf groups
   GridBarrier *d_bar_ = nullptr;
+  volatile long long *h_skipped_ = nullptr;   // steps that persistent launches left out (pinned, device-visible)
+  bool loop_failed_ = false;     // a launch was refused or timed out: per batch until SetPersistent
   int n_iaf_multi_ = 0, iaf_multi_blocks_ = 0;
   void prepare_multi();
   bool persistent_eligible() const;
@@ -425,6 +429,13 @@ class Engine {
   bool push_eligible() const;
   bool iaf_only() const;
   bool run_persistent(int steps);
+  void run_per_batch(long long n);
+  void sync_steps(const char *what);
+
+ public:
+  void set_persistent(int on);
+
+ private:
 
   template <class T> T *dalloc(size_t n);
   void free_device();
@@ -497,8 +508,8 @@ int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int persistent_blocks(int total_n, int dspan);
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
-                          const Clock *clk, int steps, GridBarrier *bar, uint64_t seed, int nblocks, int barrier_extra,
-                          cudaStream_t st);
+                          Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
+                          int barrier_extra, int gate_extra, cudaStream_t st);
 int deliver_max_pairs();
 void pack_delivery_csr_noalloc(const int *src, const int *dly, const unsigned *target, const float *weight,
                                size_t n, int n_nodes, int dspan, unsigned long long *seg_off, EdgeW *edge,

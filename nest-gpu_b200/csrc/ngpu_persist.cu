@@ -66,6 +66,23 @@ __device__ __forceinline__ void grid_arrive(unsigned *count) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
 }
 
+// The blocks wait for one another before the first of them changes anything: while another kernel
+// holds some of the GPU the launch has blocks that cannot start, and the barriers of the others
+// would run out in the middle of the steps.  Whoever waits too long (2^17 polls, 18 ms) closes
+// the gate; then no block goes on, the clock stays where it is and the engine runs the steps per
+// batch.  One compare-and-swap decides, so all blocks see the same.
+__device__ __forceinline__ void gate_enter(GridBarrier *bar, unsigned nblocks) {
+  if (atomicAdd(&bar->gate, 1u) + 1u == nblocks) atomicCAS(&bar->state, (unsigned)GATE_WAIT, (unsigned)GATE_OPEN);
+}
+__device__ __forceinline__ bool gate_wait(GridBarrier *bar) {
+  for (int polls = 0; polls < (1 << 17); polls++) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&bar->state) : "memory");
+    if (v != GATE_WAIT) return v == GATE_OPEN;
+  }
+  return atomicCAS(&bar->state, (unsigned)GATE_WAIT, (unsigned)GATE_CLOSED) == GATE_OPEN;
+}
+
 // A segment's edges e, e + stride, ..., 128 of them at a time: four loads in flight per lane
 // before their reductions.  (Eight cost registers and spills, see PersShared.)
 __device__ __forceinline__ void deliver_segment(const EdgeW *edge, double *acc, long long e0, int len, float height, int e,
@@ -105,13 +122,14 @@ __device__ __forceinline__ int slot_back(int rs, int d, int R) { return rs >= d 
 
 __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
     const DeliverArgs D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut so, const Clock *clk, int K,
-    GridBarrier *bar, uint64_t seed, int extra) {
+    GridBarrier *bar, uint64_t seed, int extra, int gate_extra) {
   extern __shared__ __align__(16) unsigned char pers_smem[];
   PersShared &S = *reinterpret_cast<PersShared *>(pers_smem);
   int *s_pref = S.pref, *s_ns = S.ns, *s_ok = S.ok;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = gridDim.x;
-  const unsigned per_bar = (unsigned)(G + extra);   // extra > 0 only in the timeout test
+  const unsigned per_bar = (unsigned)(G + extra);   // extra, gate_extra > 0 only in the tests of the failure paths
+  if (tid == 0) gate_enter(bar, (unsigned)(G + gate_extra));
   const long long t1 = clk->tidx_base + clk->it0 + 1;   // time index of the first step
   int rs = (int)(t1 % D.R);             // ring slot of the step
   int as = (int)(t1 % PERS_SLOTS);      // accumulator slot of the step
@@ -170,9 +188,11 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
     if (tid == 0) {
       S.nev = 0;
       s_ns[0] = s_ns[1] = 0;
-      if (blockIdx.x == 0) D.ring_cnt[rs] = 0;   // holds no spike of the last dmax + 1 steps
+      s_ok[0] = gate_wait(bar) ? 1 : 0;
+      if (s_ok[0] && blockIdx.x == 0) D.ring_cnt[rs] = 0;   // holds no spike of the last dmax + 1 steps
     }
     __syncthreads();
+    if (!s_ok[0]) return;
     if (warp == 0) scan_counts(D.dspan);
     __syncthreads();
     deliver_items(warp, PERS_THREADS / 32, rs0, 0, D.acc + (size_t)as * D.slot_stride);
@@ -395,6 +415,12 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
   if (tid == 0 && S.nev) atomicAdd(D.n_events, S.nev);
 }
 
+// The clock after a launch: advanced, or the steps noted for the host where the gate was closed.
+__global__ void persistent_advance_kernel(Clock *clk, int K, const GridBarrier *bar, long long *skipped) {
+  if (bar->state == GATE_OPEN) clk->it0 += K;
+  else *skipped += K;
+}
+
 // Blocks of the persistent loop for a network of `total_n` neurons and `dspan` delay groups on
 // this GPU (one neuron per neuron thread, one co-resident block per SM), 0 if it does not fit.
 int persistent_blocks(int total_n, int dspan) {
@@ -409,10 +435,11 @@ int persistent_blocks(int total_n, int dspan) {
   return per_sm >= 1 ? n_sm : 0;
 }
 
-// Cooperative launch of the persistent loop over `steps` steps.
+// Cooperative launch of the persistent loop over `steps` steps, then the clock; the number of
+// launches, or -1 where the cooperative launch is refused.
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
-                          const Clock *clk, int steps, GridBarrier *bar, uint64_t seed, int nblocks, int barrier_extra,
-                          cudaStream_t st) {
+                          Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
+                          int barrier_extra, int gate_extra, cudaStream_t st) {
   DeliverArgs d = D;
   const IafArgs *t = tab;
   const int *f = first;
@@ -422,13 +449,14 @@ int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *f
   int k = steps;
   GridBarrier *b = bar;
   uint64_t sd = seed;
-  int x = barrier_extra;
-  void *args[] = {&d, &t, &f, &ng, &s, &c, &k, &b, &sd, &x};
+  int x = barrier_extra, gx = gate_extra;
+  void *args[] = {&d, &t, &f, &ng, &s, &c, &k, &b, &sd, &x, &gx};
   if (cudaLaunchCooperativeKernel((void *)persistent_iaf_kernel, dim3(nblocks), dim3(PERS_THREADS), args,
                                   sizeof(PersShared), st) !=
       cudaSuccess)
     return -1;
-  return 1;
+  persistent_advance_kernel<<<1, 1, 0, st>>>(clk, steps, bar, skipped);
+  return 2;
 }
 
 }  // namespace ngpu

@@ -67,6 +67,8 @@ void Engine::free_device() {
   stream_ = nullptr;
   if (stream2_) cudaStreamDestroy(stream2_);
   stream2_ = nullptr;
+  if (h_skipped_) cudaFreeHost((void *)h_skipped_);
+  h_skipped_ = nullptr;
   if (ev_fork_) cudaEventDestroy(ev_fork_);
   if (ev_join_) cudaEventDestroy(ev_join_);
   ev_fork_ = ev_join_ = nullptr;
@@ -408,6 +410,12 @@ void Engine::calibrate() {
   // (the persistent loop of an iaf-only network has the arrivals of four steps open at a time)
   pers_blocks_ = 0;
   if (iaf_only()) pers_blocks_ = persistent_blocks(N, dspan_);
+  if (pers_blocks_) {
+    void *p = nullptr;
+    cuda_check(cudaHostAlloc(&p, sizeof(long long), cudaHostAllocMapped), "pinned counter");
+    h_skipped_ = (volatile long long *)p;
+    *h_skipped_ = 0;
+  }
   const size_t acc_slots = pers_blocks_ ? std::max(batch_, 4) : batch_;
   d_acc_ = dalloc<double>(n_acc_ * acc_slots);
   cuda_check(cudaMemset(d_acc_, 0, std::max<size_t>(n_acc_ * acc_slots, 1) * sizeof(double)), "memset");
@@ -1187,7 +1195,13 @@ void Engine::prepare_multi() {
 
 // The persistent step loop serves networks whose only neurons are iaf_psc_exp groups
 // (Poisson generators have no kernel of their own) and that fit it.
-bool Engine::persistent_eligible() const { return !push_ && pers_blocks_ > 0; }
+bool Engine::persistent_eligible() const { return !push_ && pers_blocks_ > 0 && !loop_failed_; }
+
+void Engine::set_persistent(int on) {
+  persistent = on;
+  loop_failed_ = false;
+  invalidate_graphs();
+}
 
 // Networks with a minimum delay of one step run in the persistent loop by themselves: a step is
 // then two short dependent launches otherwise (ngpu_persist.cu has both times).  With longer
@@ -1224,20 +1238,34 @@ bool Engine::iaf_only() const {
 
 // `steps` steps in one cooperative launch of the persistent loop, then the clock advance; false if
 // the launch was refused and the loop was the engine's own choice (the caller goes on per batch).
+// A launch whose blocks cannot all start runs no step and notes them in *h_skipped_.
 bool Engine::run_persistent(int steps) {
   cuda_check(cudaMemsetAsync(d_bar_, 0, sizeof(GridBarrier), stream_), "barrier reset");
-  const int r = launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_,
-                                      steps, d_bar_, kernel_seed, pers_blocks_, barrier_extra, stream_);
+  const int r = loop_start_test == 1 ? -1 :
+      launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_, steps, d_bar_,
+                            (long long *)h_skipped_, kernel_seed, pers_blocks_, barrier_extra, loop_start_test == 2,
+                            stream_);
   if (r < 0 && persistent < 0) {
     cudaGetLastError();
-    persistent = 0;
+    loop_failed_ = true;
+    invalidate_graphs();
     return false;
   }
   if (r < 0) throw NgpuError(std::string("cooperative launch of the persistent step loop failed: ") +
                              cudaGetErrorString(cudaGetLastError()));
-  launch_clock_advance(d_clk_, steps, stream_);
-  n_launch_ += 2;
+  n_launch_ += r;
   return true;
+}
+
+// Waits for the stream, then runs per batch what persistent launches left out.
+void Engine::sync_steps(const char *what) {
+  cuda_check(cudaStreamSynchronize(stream_), what);
+  if (!h_skipped_ || *h_skipped_ == 0) return;
+  const long long n = *h_skipped_;
+  *h_skipped_ = 0;
+  run_per_batch(n);
+  if (ev_b_) cuda_check(cudaEventRecord(ev_b_, stream_), "event");   // the device time of the call includes them
+  cuda_check(cudaStreamSynchronize(stream_), what);
 }
 
 void Engine::ensure_record_window(long long rows) {
@@ -1299,13 +1327,40 @@ void Engine::run_batches_partitioned(long long n) {
 // Steps per launch of the persistent loop: launch and prologue are a few steps' time.
 constexpr long long PERS_STEPS = 2000;
 
+// n steps in CUDA graphs of per-batch launches.
+void Engine::run_per_batch(long long n) {
+  const int M = batch_;
+  const int K = std::max(M, (std::max(1, graph_steps) / M) * M);   // steps per graph
+  while (n > 0) {
+    const int steps = (int)std::min<long long>(K, n);
+    auto itg = graphs_.find(steps);
+    if (itg == graphs_.end()) {
+      prepare_multi();
+      cudaGraph_t graph;
+      cuda_check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
+      capturing_ = true;
+      capture_count_ = 0;
+      for (int k0 = 0; k0 < steps; k0 += M) launch_batch(k0, std::min(M, steps - k0), nullptr);
+      count_launch(launch_clock_advance(d_clk_, steps, stream_));
+      capturing_ = false;
+      graph_nodes_[steps] = capture_count_;
+      cuda_check(cudaStreamEndCapture(stream_, &graph), "capture");
+      cudaGraphExec_t exec;
+      cuda_check(cudaGraphInstantiate(&exec, graph, 0), "instantiate");
+      cudaGraphDestroy(graph);
+      itg = graphs_.emplace(steps, exec).first;
+    }
+    cuda_check(cudaGraphLaunch(itg->second, stream_), "graph launch");
+    n_launch_ += graph_nodes_[steps];
+    n -= steps;
+  }
+}
+
 void Engine::run_steps(long long n) {
   if (part_world_ > 1) {
     run_batches_partitioned(n);
     return;
   }
-  const int M = batch_;
-  const int K = std::max(M, (std::max(1, graph_steps) / M) * M);   // steps per graph
   long long window = n;
   const long long REC_WINDOW = 10000;
   if (rec_ncol_) {
@@ -1314,40 +1369,19 @@ void Engine::run_steps(long long n) {
   }
   bool pers = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(n));
   if (pers) prepare_multi();
-  long long done = 0;
-  while (done < n) {
+  for (long long done = 0; done < n;) {
     const long long w = std::min(window, n - done);
     long long left = w;
-    while (left > 0) {
-      if (pers) {
-        const int steps = (int)std::min<long long>(PERS_STEPS, left);
-        pers = run_persistent(steps);
-        if (pers) left -= steps;
-        continue;
-      }
-      const int steps = (int)std::min<long long>(K, left);
-      auto itg = graphs_.find(steps);
-      if (itg == graphs_.end()) {
-        prepare_multi();
-        cudaGraph_t graph;
-        cuda_check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture");
-        capturing_ = true;
-        capture_count_ = 0;
-        for (int k0 = 0; k0 < steps; k0 += M) launch_batch(k0, std::min(M, steps - k0), nullptr);
-        count_launch(launch_clock_advance(d_clk_, steps, stream_));
-        capturing_ = false;
-        graph_nodes_[steps] = capture_count_;
-        cuda_check(cudaStreamEndCapture(stream_, &graph), "capture");
-        cudaGraphExec_t exec;
-        cuda_check(cudaGraphInstantiate(&exec, graph, 0), "instantiate");
-        cudaGraphDestroy(graph);
-        itg = graphs_.emplace(steps, exec).first;
-      }
-      cuda_check(cudaGraphLaunch(itg->second, stream_), "graph launch");
-      n_launch_ += graph_nodes_[steps];
-      left -= steps;
+    while (pers && left > 0) {
+      const int steps = (int)std::min<long long>(PERS_STEPS, left);
+      pers = run_persistent(steps);
+      if (pers) left -= steps;
     }
-    if (rec_ncol_) drain_records(w);
+    run_per_batch(left);
+    if (rec_ncol_) {
+      sync_steps("records");
+      drain_records(w);
+    }
     done += w;
   }
 }
@@ -1418,7 +1452,8 @@ void Engine::check_status() {
     const unsigned keep = st & ~ST_BARRIER_TIMEOUT;
     cuda_check(cudaMemcpy(d_status_, &keep, sizeof(unsigned), cudaMemcpyHostToDevice), "status");
     status_seen_ &= ~ST_BARRIER_TIMEOUT;
-    persistent = 0;
+    loop_failed_ = true;
+    invalidate_graphs();
     cuda_check(cudaMemset(d_acc_, 0, n_acc_ * (size_t)std::max(batch_, 4) * sizeof(double)), "memset");
     throw NgpuError("a grid barrier of the persistent step loop timed out; the simulation state is invalid "
                     "(the engine falls back to per-batch launches)");
@@ -1478,7 +1513,7 @@ void Engine::start_simulation() {
 
 void Engine::end_simulation() {
   if (!in_sim_) return;
-  cuda_check(cudaStreamSynchronize(stream_), "end of simulation");
+  sync_steps("end of simulation");
   drain_rec_spike_times();
   if (it_ > 0) neural_time_ = neur_t0_ + (double)dt * (double)it_;
   in_sim_ = false;
@@ -1494,7 +1529,7 @@ void Engine::simulation_step() {
   // reference shows
   run_steps(1);
   it_ += 1;
-  cuda_check(cudaStreamSynchronize(stream_), "step");
+  sync_steps("step");
   neural_time_ = neur_t0_ + (double)dt * (double)it_;
 }
 

@@ -37,8 +37,11 @@ enum Status : unsigned {
 };
 
 // Barrier state of the persistent step loop (device memory, zero-initialised).
+enum GateState : unsigned { GATE_WAIT = 0, GATE_OPEN = 1, GATE_CLOSED = 2 };
 struct GridBarrier {
   unsigned count;        // arrivals since the launch
+  unsigned gate;         // blocks that have started
+  unsigned state;        // GateState: all blocks run, or one of them gave up waiting for the others
 };
 
 // Simulation clock in device memory.  A CUDA graph covers a fixed number of steps

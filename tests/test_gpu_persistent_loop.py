@@ -124,3 +124,63 @@ def test_two_networks_in_two_threads():
     for key in (0, 1):
         assert alone[key][0].sum() > 0
         assert all(np.array_equal(x, y) for x, y in zip(alone[key], both[key]))
+
+
+def _count_launches(fn):
+    l0 = ngpu.GetLaunchCount()
+    fn()
+    return ngpu.GetLaunchCount() - l0
+
+
+@pytest.mark.parametrize("forced", [None, True])
+def test_blocks_that_cannot_all_start(forced):
+    """A launch whose blocks do not all start (here its gate waits for one block too many) changes
+    nothing and its steps run per batch: counts, potentials, records and the time are those of the
+    per-batch kernels alone, spikes in flight included, and the next call is a loop again."""
+    def run(modes):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 400, 0.1, 2.0)
+        rec = ngpu.CreateRecord("", ["V_m_rel", "spike"], [pops[0][0], pops[1][3]], [0, 0])
+        launches = []
+        for m in modes:
+            if modes[0] is None:
+                ngpu.SetPersistent(False)
+            elif forced:
+                ngpu.SetPersistent(True)
+            ngpu._lib.NGPU_TestLoopStart(m or 0)
+            launches.append(_count_launches(lambda: ngpu.Simulate(4.0)))
+            if forced:
+                ngpu.SimulationStep()
+                ngpu.EndSimulation()
+        ngpu._lib.NGPU_TestLoopStart(0)
+        return _state(ngpu, pops) + (ngpu.GetStats()["n_events"], np.asarray(ngpu.GetRecordData(rec))), launches
+    want, _ = run([None] * 4)
+    got, launches = run([0, 2, 0, 2])
+    assert want[0].sum() > 50 and all(np.array_equal(x, y) for x, y in zip(got, want))
+    assert launches[0] == launches[2] == 2 and min(launches[1], launches[3]) > 2
+    assert ngpu.GetStats()["status"] == 0
+
+
+def test_refused_launch():
+    """A refused cooperative launch: the engine's own choice goes on per batch and says so, a loop
+    that was asked for fails; SetPersistent brings the loop back."""
+    ngpu.SetPersistent(False)
+    pops = _net(ngpu, 400, 0.1, 2.0)
+    ngpu.Simulate(8.0)
+    want = _state(ngpu, pops)
+    ngpu.Reset()
+    ngpu.SetVerbosityLevel(0)
+    pops = _net(ngpu, 400, 0.1, 2.0)
+    ngpu.Simulate(4.0)
+    assert ngpu.GetLaunchMapping()["persistent"] == 1
+    ngpu._lib.NGPU_TestLoopStart(1)
+    ngpu.Simulate(4.0)
+    assert all(np.array_equal(x, y) for x, y in zip(_state(ngpu, pops), want))
+    assert ngpu.GetLaunchMapping()["persistent"] == 0
+    ngpu.SetPersistent(True)
+    with pytest.raises(ValueError, match="cooperative launch"):
+        ngpu.Simulate(4.0)
+    ngpu._lib.NGPU_TestLoopStart(0)
+    ngpu.EndSimulation()
+    assert _count_launches(lambda: ngpu.Simulate(4.0)) == 2
