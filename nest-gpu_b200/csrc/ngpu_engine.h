@@ -506,7 +506,7 @@ long long check_rounded_ops();
 // STDP (ngpu_stdp.cu)
 int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
-int persistent_blocks(int total_n, int dspan);
+int persistent_blocks(long long n_iaf, int dspan);
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
                           Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
                           int barrier_extra, int gate_extra, cudaStream_t st);

@@ -421,13 +421,14 @@ __global__ void persistent_advance_kernel(Clock *clk, int K, const GridBarrier *
   else *skipped += K;
 }
 
-// Blocks of the persistent loop for a network of `total_n` neurons and `dspan` delay groups on
-// this GPU (one neuron per neuron thread, one co-resident block per SM), 0 if it does not fit.
-int persistent_blocks(int total_n, int dspan) {
+// Blocks of the persistent loop for a network of `n_iaf` iaf_psc_exp neurons and `dspan` delay
+// groups on this GPU (one neuron per neuron thread, one co-resident block per SM), 0 if it does
+// not fit.
+int persistent_blocks(long long n_iaf, int dspan) {
   int dev = 0, n_sm = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  if (dspan > PERS_MAX_SPAN || (long long)total_n > (long long)n_sm * PERS_NEURON) return 0;
+  if (dspan > PERS_MAX_SPAN || n_iaf > (long long)n_sm * PERS_NEURON) return 0;
   if (cudaFuncSetAttribute(persistent_iaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersShared)) !=
       cudaSuccess)
     return 0;

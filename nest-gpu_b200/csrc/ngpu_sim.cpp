@@ -409,7 +409,12 @@ void Engine::calibrate() {
   if (dspan_ * batch_ > deliver_max_pairs()) batch_ = std::max(1, deliver_max_pairs() / dspan_);
   // (the persistent loop of an iaf-only network has the arrivals of four steps open at a time)
   pers_blocks_ = 0;
-  if (iaf_only()) pers_blocks_ = persistent_blocks(N, dspan_);
+  if (iaf_only()) {
+    long long n_iaf = 0;   // (generators take no thread of the loop)
+    for (auto &g : groups_)
+      if (g.model == M_IAF_PSC_EXP) n_iaf += g.n;
+    pers_blocks_ = persistent_blocks(n_iaf, dspan_);
+  }
   if (pers_blocks_) {
     void *p = nullptr;
     cuda_check(cudaHostAlloc(&p, sizeof(long long), cudaHostAllocMapped), "pinned counter");

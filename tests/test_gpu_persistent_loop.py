@@ -44,6 +44,12 @@ def _state(api, pops):
             np.concatenate([np.asarray(api.GetStatus(p, "V_m_rel"), dtype=np.float32).ravel() for p in pops]))
 
 
+def _count_launches(fn):
+    l0 = ngpu.GetLaunchCount()
+    fn()
+    return ngpu.GetLaunchCount() - l0
+
+
 @pytest.mark.parametrize("n,lo,hi", [(2, 0.1, 0.1), (147, 0.1, 0.2), (149, 0.1, 3.0), (1000, 0.2, 0.2), (1000, 0.2, 1.7),
                                      (700, 0.3, 2.0), (300, 1.5, 1.5), (900, 0.1, 19.2)])
 def test_delay_ranges_match_oracle(n, lo, hi):
@@ -52,7 +58,7 @@ def test_delay_ranges_match_oracle(n, lo, hi):
     o = orc.Oracle()
     opops = _net(o, n, lo, hi)
     for t in (20.0, 0.1, 0.2, 0.3, 13.7):
-        ngpu.Simulate(t)
+        assert _count_launches(lambda: ngpu.Simulate(t)) == 2
         o.Simulate(t)
     c, v = _state(ngpu, pops)
     co, vo = _state(o, opops)
@@ -61,17 +67,19 @@ def test_delay_ranges_match_oracle(n, lo, hi):
     assert ngpu.GetStats()["n_events"] == o.NEvents() and ngpu.GetStats()["status"] == 0
 
 
-@pytest.mark.parametrize("n,hi", [(576 * 148, 1.0), (576 * 148 + 1, 1.0), (400, 19.3)])
-def test_capacity_and_what_lies_beyond_it(n, hi):
-    """The largest network of the loop, one neuron more, and one delay group too many (the last
-    two run in the per-batch kernels) equal the per-batch kernels."""
+@pytest.mark.parametrize("n,hi,loop", [(576 * 148, 1.0, True), (576 * 148 + 1, 1.0, False), (400, 19.2, True),
+                                       (400, 19.3, False)])
+def test_capacity_and_what_lies_beyond_it(n, hi, loop):
+    """The largest network of the loop (its two generators take no thread), one neuron more, and
+    one delay group too many (these two run in the per-batch kernels) equal the per-batch kernels."""
     res = []
     for pers in (True, False):
         ngpu.Reset()
         ngpu.SetVerbosityLevel(0)
         ngpu.SetPersistent(pers)
         pops = _net(ngpu, n, 0.1, hi, k=5)
-        ngpu.Simulate(12.0)
+        launches = _count_launches(lambda: ngpu.Simulate(12.0))
+        assert (launches == 2) == (pers and loop)
         res.append(_state(ngpu, pops) + (ngpu.GetStats()["n_events"],))
     assert res[0][0].sum() > 0 and all(np.array_equal(x, y) for x, y in zip(*res))
 
@@ -126,12 +134,6 @@ def test_two_networks_in_two_threads():
         assert all(np.array_equal(x, y) for x, y in zip(alone[key], both[key]))
 
 
-def _count_launches(fn):
-    l0 = ngpu.GetLaunchCount()
-    fn()
-    return ngpu.GetLaunchCount() - l0
-
-
 @pytest.mark.parametrize("forced", [None, True])
 def test_blocks_that_cannot_all_start(forced):
     """A launch whose blocks do not all start (here its gate waits for one block too many) changes
@@ -184,3 +186,19 @@ def test_refused_launch():
     ngpu._lib.NGPU_TestLoopStart(0)
     ngpu.EndSimulation()
     assert _count_launches(lambda: ngpu.Simulate(4.0)) == 2
+
+
+def test_generators_take_no_place_in_the_loop():
+    """More generator nodes than the loop has threads, beside a network that fits it."""
+    def run(pers):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 300, 0.1, 2.0)
+        ngpu.Create("poisson_generator", 576 * 148)
+        if not pers:
+            ngpu.SetPersistent(False)
+        launches = _count_launches(lambda: ngpu.Simulate(8.0))
+        return _state(ngpu, pops), launches
+    (got, launches), (want, _) = run(True), run(False)
+    assert launches == 2
+    assert want[0].sum() > 0 and all(np.array_equal(x, y) for x, y in zip(got, want))
