@@ -411,7 +411,9 @@ int NGPU_TestTensorWaitTimeout(int on);
    network, after 4 x `steps` warm-up steps, times `steps` simulation steps per candidate of the
    update block size, the update kernel variant, the delivery lane group, the delivery grid and
    the RK5 step budget, each candidate twice (forward and reverse order), in a coordinate
-   descent of two passes, and keeps the fastest.  The trials are ordinary simulation steps, so
+   descent of two passes, and keeps the fastest.  The descent starts from what is set, and what
+   is automatic stays automatic where no value beats it; a failed call leaves the settings as they
+   were.  The trials are ordinary simulation steps, so
    the network advances by them.  Returns the number of trials (-1 on error) and the chosen
    values. */
 int NGPU_Autotune(int steps, int *update_threads, int *deliver_group, int *deliver_blocks,

@@ -141,7 +141,9 @@ class Engine {
   int update_occupancy = -1;      // 1, 2: register-capped aeif update kernel (-1: by aeif_mapping)
   int update_trial_iter = -1;     // 1: aeif update kernel advances one RK5 trial per iteration (-1: by
                                   // aeif_mapping)
-  int persistent = -1;            // iaf-only networks: persistent cooperative step loop (-1: by persistent_auto)
+  int persistent = -1;            // iaf-only networks: persistent cooperative step loop (-1: by persistent_auto,
+                                  // LOOP_LONG_CALLS: as Autotune found, for calls that are long enough)
+  static constexpr int LOOP_LONG_CALLS = 2;
   int launch_pdl = -1;            // programmatic dependent launch of the batch kernels (-1: one-step batches)
   int loop_start_test = 0;        // test hook: 1: the persistent loop's launch counts as refused, 2: its gate
                                   // waits for one block more than the launch has
@@ -425,6 +427,7 @@ class Engine {
   void prepare_multi();
   bool persistent_eligible() const;
   bool persistent_auto(long long steps) const;
+  bool use_loop(long long steps) const;
   int pers_blocks_ = 0;          // blocks of the persistent loop (0: it cannot run this network)
   bool push_eligible() const;
   bool iaf_only() const;

@@ -868,8 +868,7 @@ Engine::Mapping Engine::mapping_in_use() const {
   A.hi = big->hi;
   aeif_mapping(*big, A);
   Mapping m{A.threads, A.occupancy, A.trial_iter, A.budget > 0 ? A.budget - batch_ : 0, 0};
-  if (!calibrated_) m.persistent = persistent > 0;
-  else m.persistent = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(1LL << 30));
+  m.persistent = calibrated_ ? use_loop(1LL << 30) : persistent > 0;
   return m;
 }
 
@@ -1218,11 +1217,20 @@ void Engine::set_persistent(int on) {
 // 109, 184 and 337 us) per batch, so the line lies at four steps.  Neurons with several
 // generators each stay with the per-batch kernels, where poisson_multi_kernel spreads their draws
 // over the GPU.
+constexpr long long LOOP_MIN_STEPS = 4;
+
 bool Engine::persistent_auto(long long steps) const {
-  if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < 4) return false;
+  if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < LOOP_MIN_STEPS) return false;
   for (auto &g : groups_)
     if (g.d_pin_tgt) return false;
   return true;
+}
+
+// Does a call of `steps` steps run in the persistent loop?
+bool Engine::use_loop(long long steps) const {
+  if (persistent < 0) return persistent_auto(steps);
+  if (persistent == LOOP_LONG_CALLS && steps < LOOP_MIN_STEPS) return false;
+  return persistent > 0 && persistent_eligible();
 }
 
 // Delivery at emission serves the same networks as the persistent loop.
@@ -1250,7 +1258,7 @@ bool Engine::run_persistent(int steps) {
       launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_, steps, d_bar_,
                             (long long *)h_skipped_, kernel_seed, pers_blocks_, barrier_extra, loop_start_test == 2,
                             stream_);
-  if (r < 0 && persistent < 0) {
+  if (r < 0 && persistent != 1) {
     cudaGetLastError();
     loop_failed_ = true;
     invalidate_graphs();
@@ -1372,7 +1380,7 @@ void Engine::run_steps(long long n) {
     window = std::min<long long>(n, REC_WINDOW);
     ensure_record_window(window);
   }
-  bool pers = persistent > 0 ? persistent_eligible() : (persistent < 0 && persistent_auto(n));
+  bool pers = use_loop(n);
   if (pers) prepare_multi();
   for (long long done = 0; done < n;) {
     const long long w = std::min(window, n - done);
@@ -1689,14 +1697,36 @@ int Engine::autotune(int steps, std::vector<std::pair<std::string, double>> *log
       single("rk5_budget", &rk5_budget, {0, 1, 2, 4, 8}),
       single("programmatic_launch", &launch_pdl, {0, 1}),
   };
-  if (persistent_eligible()) knobs.insert(knobs.begin(), single("persistent", &persistent, {0, 1}));
+  // (the loop in the form that leaves short calls to the per-batch kernels, unless it was forced)
+  if (persistent_eligible())
+    knobs.insert(knobs.begin(), single("persistent", &persistent, {0, persistent == 1 ? 1 : LOOP_LONG_CALLS}));
+  // What is automatic stays so unless an explicit value beats it: the automatic mapping is chosen
+  // group by group, which no value for all groups can express.  A value that is what the automatic
+  // choice comes to for every group is not timed beside it.
+  auto is_automatic = [&](const int *var, int v) {
+    if (var == &persistent) return persistent < 0 && (v != 0) == persistent_auto(steps);
+    if (var == &update_threads ? update_threads > 0
+                               : (var != &update_occupancy && var != &update_trial_iter && var != &rk5_budget) || *var >= 0)
+      return false;
+    for (auto &g : groups_) {
+      if (!is_aeif(g.model) || g.hi <= g.lo) continue;
+      AeifArgs A;
+      std::memset(&A, 0, sizeof(A));
+      A.lo = g.lo;
+      A.hi = g.hi;
+      aeif_mapping(g, A);
+      const int budget = A.budget > 0 ? A.budget - batch_ : 0;
+      if (v != (var == &update_threads ? A.threads : var == &update_occupancy ? A.occupancy
+                : var == &update_trial_iter ? A.trial_iter : budget))
+        return false;
+    }
+    return true;
+  };
+  std::vector<std::pair<int *, int>> before{{&deliver_blocks_req, deliver_blocks_req}};
+  for (auto &k : knobs)
+    for (int *p : k.vars)
+      if (p != &deliver_blocks_req) before.push_back({p, *p});
   if (deliver_blocks_req <= 0) deliver_blocks_req = base;
-  // the descent starts from explicit values where the mapping was automatic
-  if (update_threads <= 0) update_threads = 128;
-  if (update_occupancy < 0) update_occupancy = 0;
-  if (update_trial_iter < 0) update_trial_iter = 0;
-  if (rk5_budget < 0) rk5_budget = 4;
-  if (persistent < 0) persistent = persistent_auto(steps) ? 1 : 0;
   const float t = (float)steps * dt;
   auto trial = [&]() {
     invalidate_graphs();
@@ -1721,7 +1751,8 @@ int Engine::autotune(int steps, std::vector<std::pair<std::string, double>> *log
         for (int *p : k.vars) cur.push_back(*p);
         cand.push_back(cur);
         for (auto &c : k.cand)
-          if (c != cur) cand.push_back(c);
+          if (c != cur && !(c.size() == 1 && is_automatic(k.vars[0], c[0]))) cand.push_back(c);
+        if (cand.size() == 1) continue;
         std::vector<double> best_ms(cand.size(), 1e300);
         for (int rep = 0; rep < 2; rep++) {
           for (size_t u = 0; u < cand.size(); u++) {
@@ -1745,6 +1776,8 @@ int Engine::autotune(int steps, std::vector<std::pair<std::string, double>> *log
     }
   } catch (...) {
     verbosity = verb;
+    for (auto &b : before) *b.first = b.second;
+    invalidate_graphs();
     throw;
   }
   verbosity = verb;

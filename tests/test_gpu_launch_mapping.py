@@ -49,3 +49,47 @@ def test_persistent_loop_in_use_is_reported(n, lo, hi, forced, want):
     l0 = ngpu.GetLaunchCount()
     ngpu.Simulate(2.0)
     assert (ngpu.GetLaunchCount() - l0 == 2) == bool(want)
+
+
+def test_autotune_leaves_short_calls_to_the_per_batch_kernels():
+    """A single step after Autotune goes the way it goes without it: the loop that wins on long
+    calls costs more there."""
+    from workloads import microcircuit
+    microcircuit(ngpu, scale=0.03)
+    ngpu.Simulate(5.0)
+
+    def launches(fn):
+        l0 = ngpu.GetLaunchCount()
+        fn()
+        return ngpu.GetLaunchCount() - l0
+    before = launches(ngpu.SimulationStep)
+    ngpu.EndSimulation()
+    assert ngpu.Autotune(50)["persistent"] == 1 and launches(lambda: ngpu.Simulate(2.0)) == 2
+    assert launches(ngpu.SimulationStep) == before > 2
+    ngpu.EndSimulation()
+
+
+def test_autotune_keeps_what_is_automatic():
+    """Settings without influence on a network (here the aeif ones, without an aeif group) stay as
+    they were."""
+    _iaf(500, 1.0, 1.5)
+    ngpu.Simulate(2.0)
+    keys = ["update_threads", "update_occupancy", "update_trial_iter", "rk5_budget"]
+    before = ngpu.GetLaunchMapping()
+    after = ngpu.Autotune(20)
+    assert [before[k] for k in keys] == [after[k] for k in keys]
+
+
+def test_failed_autotune_leaves_the_settings():
+    """A trial that fails (its barriers wait for one block too many) ends the call with the
+    settings of before; the loop itself stays off, as after any such failure."""
+    _iaf(500)
+    ngpu.Simulate(2.0)
+    before = ngpu.GetLaunchMapping()
+    ngpu._lib.NGPU_TestBarrierTimeout(1)
+    with pytest.raises(ValueError, match="timed out"):
+        ngpu.Autotune(20)
+    ngpu._lib.NGPU_TestBarrierTimeout(0)
+    after = ngpu.GetLaunchMapping()
+    assert before.pop("persistent") == 1 and after.pop("persistent") == 0
+    assert before == after
