@@ -429,6 +429,7 @@ class Engine {
   bool persistent_auto(long long steps) const;
   bool use_loop(long long steps) const;
   int pers_blocks_ = 0;          // blocks of the persistent loop (0: it cannot run this network)
+  double own_edges_ = 0.0;       // mean number of a source's edges that its own block delivers there
   bool push_eligible() const;
   bool iaf_only() const;
   bool run_persistent(int steps);
@@ -510,6 +511,7 @@ long long check_rounded_ops();
 int launch_stdp_forward(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int launch_stdp_reverse(const StdpArgs &A, const Clock *clk, int k0, cudaStream_t st);
 int persistent_blocks(long long n_iaf, int dspan);
+long long persistent_own_edges(const long long *ev_off, int n_nodes, int dspan, unsigned long long *d_sum);
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
                           Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
                           int barrier_extra, int gate_extra, cudaStream_t st);

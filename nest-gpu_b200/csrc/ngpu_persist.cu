@@ -421,6 +421,26 @@ __global__ void persistent_advance_kernel(Clock *clk, int K, const GridBarrier *
   else *skipped += K;
 }
 
+// Edges of total delay one and two steps (the first `groups` delay groups of every node).
+__global__ void first_edges_kernel(const long long *ev_off, int n_nodes, int dspan, int groups, unsigned long long *sum) {
+  unsigned long long s = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
+    const long long *off = ev_off + (size_t)i * dspan;
+    s += (unsigned long long)(off[groups] - off[0]);
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(sum, s);
+}
+
+// `d_sum`: a zeroed counter on the device.  -1: it could not run.
+long long persistent_own_edges(const long long *ev_off, int n_nodes, int dspan, unsigned long long *d_sum) {
+  first_edges_kernel<<<std::min((n_nodes + 255) / 256, 592), 256>>>(ev_off, n_nodes, dspan, std::min(dspan, 2), d_sum);
+  unsigned long long h = 0;
+  if (cudaGetLastError() != cudaSuccess) return -1;
+  if (cudaMemcpy(&h, d_sum, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+  return (long long)h;
+}
+
 // Blocks of the persistent loop for a network of `n_iaf` iaf_psc_exp neurons and `dspan` delay
 // groups on this GPU (one neuron per neuron thread, one co-resident block per SM), 0 if it does
 // not fit.

@@ -420,6 +420,14 @@ void Engine::calibrate() {
     cuda_check(cudaHostAlloc(&p, sizeof(long long), cudaHostAllocMapped), "pinned counter");
     h_skipped_ = (volatile long long *)p;
     *h_skipped_ = 0;
+    own_edges_ = 0.0;
+    if (dmin_ == 0 && n_src_out > 0) {
+      unsigned long long *d_sum = dalloc<unsigned long long>(1);
+      cuda_check(cudaMemset(d_sum, 0, sizeof(*d_sum)), "memset");
+      const long long sum = persistent_own_edges(d_ev_off_, N, dspan_, d_sum);
+      if (sum < 0) throw NgpuError("counting the edges of the first delays failed");
+      own_edges_ = (double)sum / n_src_out;
+    }
   }
   const size_t acc_slots = pers_blocks_ ? std::max(batch_, 4) : batch_;
   d_acc_ = dalloc<double>(n_acc_ * acc_slots);
@@ -1217,10 +1225,18 @@ void Engine::set_persistent(int on) {
 // 109, 184 and 337 us) per batch, so the line lies at four steps.  Neurons with several
 // generators each stay with the per-batch kernels, where poisson_multi_kernel spreads their draws
 // over the GPU.
+// A spiking neuron's edges of total delay one and two steps are delivered by its own block, two
+// warps a spike, while the delivery kernel cuts long segments into parts over the GPU.  us per step,
+// loop / per batch, 20,000 neurons with all delays one step: 1000 edges a source 5.7 / 8.8, 1500
+// 7.0 / 8.7, 2000 8.3 / 9.0, 2500 9.6 / 9.8, 3000 10.8 / 9.8, 10,000 29.2 / 13.5; one and two steps:
+// 1500 5.7 / 8.9, 3000 8.8 / 9.3, 4000 11.0 / 9.7, 8000 19.7 / 11.6; one to three, 6000 (4000 of
+// them in the first two) 12.2 / 10.7.  With more neurons the loop keeps its lead for longer (80,000
+// neurons, 3000: 12.7 / 15.0); the line lies where it is lost first.
 constexpr long long LOOP_MIN_STEPS = 4;
+constexpr double LOOP_OWN_EDGES = 2500.0;
 
 bool Engine::persistent_auto(long long steps) const {
-  if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < LOOP_MIN_STEPS) return false;
+  if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < LOOP_MIN_STEPS || own_edges_ > LOOP_OWN_EDGES) return false;
   for (auto &g : groups_)
     if (g.d_pin_tgt) return false;
   return true;

@@ -1,5 +1,6 @@
 """The launch mapping that the engine chooses where no call sets one: what GetLaunchMapping reports
 of it, and how Autotune starts from it and leaves it."""
+import numpy as np
 import pytest
 
 import nestgpu as ngpu
@@ -93,3 +94,28 @@ def test_failed_autotune_leaves_the_settings():
     after = ngpu.GetLaunchMapping()
     assert before.pop("persistent") == 1 and after.pop("persistent") == 0
     assert before == after
+
+
+@pytest.mark.parametrize("k,hi,loop", [(2400, 0.1, True), (2600, 0.1, False), (2400, 0.2, True), (2600, 0.2, False),
+                                       (3300, 0.3, True), (4200, 0.3, False)])
+def test_long_first_segments_stay_with_the_per_batch_kernels(k, hi, loop):
+    """Edges of one and two steps' delay are delivered by the spiking neuron's own block: above 2500 of
+    them a source the loop is not chosen.  The results are the same either way."""
+    def run(setting):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        n = ngpu.Create("iaf_psc_exp", 100)
+        ngpu.SetStatus(n, "I_e", 600.0)
+        ngpu.ConnectFixedIndegreeGPU(n, n, k, 0.01, 0.1, hi, receptor=0, seed=1)
+        ngpu.ActivateSpikeCount(n)
+        if setting is not None:
+            ngpu.SetPersistent(setting)
+        ngpu.Simulate(1.0)
+        m = ngpu.GetLaunchMapping()["persistent"]
+        ngpu.Simulate(30.0)
+        return m, np.asarray(ngpu.GetStatus(n, "spike_count")).ravel(), np.asarray(ngpu.GetStatus(n, "V_m_rel")).ravel()
+    got, off, on = run(None), run(False), run(True)
+    assert (got[0], off[0], on[0]) == (int(loop), 0, 1)
+    assert got[1].sum() > 0
+    for other in (off, on):
+        assert np.array_equal(got[1], other[1]) and np.array_equal(got[2], other[2])
