@@ -75,6 +75,9 @@ __device__ __noinline__ unsigned long long push_out_edges(const PushOut &po, int
   return (unsigned long long)(s1 - s0);
 }
 
+// AHEAD: the input of the step after next is on its way while a step is integrated; else the step's
+// own input is asked for as the step begins.  launch_iaf has the line between the two.
+template <bool AHEAD>
 __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so, const Clock *clk, int k0,
                                            int M, int i) {
   const int n = A.n;
@@ -84,14 +87,16 @@ __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so,
   const long long rec_it0 = cl.rec_it0;
   PoissonCache pc;
   poisson_cache_load(A.in, i, pc);
-  // the input of the step after next is on its way while a step is integrated
   double apf[2], next[2];
-  acc_prefetch<2>(apf, 2, n, i, A.in, 0);
-  acc_prefetch<2>(next, M > 1 ? 2 : 0, n, i, A.in, 1);
+  if constexpr (AHEAD) {
+    acc_prefetch<2>(apf, 2, n, i, A.in, 0);
+    acc_prefetch<2>(next, M > 1 ? 2 : 0, n, i, A.in, 1);
+  }
   for (int m = 0; m < M; m++) {
     const StepT t = step_at(cl, k0, m, A.dt);
     double after[2];
-    acc_prefetch<2>(after, m + 2 < M ? 2 : 0, n, i, A.in, m + 2);
+    if constexpr (AHEAD) acc_prefetch<2>(after, m + 2 < M ? 2 : 0, n, i, A.in, m + 2);
+    else acc_prefetch<2>(apf, 2, n, i, A.in, m);
     if (iaf_step(q)) push_spike(so, A.srec, A.i0 + i, i, 1.0f, t.tidx, t.tnow);
     if (A.rec.first) {
       const float yr[4] = {q.Iex, q.Iin, q.V, q.refr};
@@ -100,10 +105,12 @@ __device__ __forceinline__ void iaf_neuron(const IafArgs &A, const SpikeOut &so,
     double in[2];
     step_inputs_pf<2>(in, apf, 2, n, i, A.in, pc, m, t.tidx, t.tnow);
     iaf_fold(q, in);
-    apf[0] = next[0];
-    apf[1] = next[1];
-    next[0] = after[0];
-    next[1] = after[1];
+    if constexpr (AHEAD) {
+      apf[0] = next[0];
+      apf[1] = next[1];
+      next[0] = after[0];
+      next[1] = after[1];
+    }
   }
   iaf_store(A, i, q);
 }
@@ -186,11 +193,14 @@ __device__ __forceinline__ void iaf_neuron_push(const IafArgs &A, const SpikeOut
   if (threadIdx.x == 0 && nev) atomicAdd(po.n_events, nev);
 }
 
-__global__ void __launch_bounds__(256, 3) iaf_batch_kernel(const IafArgs A, const SpikeOut so,
-                                                        const Clock *clk, int k0, int M) {
+// TB = 64 is not capped to three 256-thread blocks' registers: with the cap the loads two steps ahead
+// spill 52 bytes per thread.
+template <int TB, bool AHEAD>
+__global__ void __launch_bounds__(TB, TB == 64 ? 1 : 3) iaf_batch_kernel(const IafArgs A, const SpikeOut so,
+                                                                       const Clock *clk, int k0, int M) {
   pdl_enter();
   const int i = A.lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < A.hi) iaf_neuron(A, so, clk, k0, M, i);
+  if (i < A.hi) iaf_neuron<AHEAD>(A, so, clk, k0, M, i);
 }
 
 // Delivery at emission: every thread of the block runs the step loop.
@@ -219,7 +229,7 @@ __global__ void __launch_bounds__(256, 3) iaf_multi_kernel(const IafArgs *tab, c
   }
   const IafArgs &A = tab[lo];
   const int i = A.lo + ((int)blockIdx.x - blk0[lo]) * blockDim.x + threadIdx.x;
-  if (i < A.hi) iaf_neuron(A, so, clk, k0, M, i);
+  if (i < A.hi) iaf_neuron<false>(A, so, clk, k0, M, i);
 }
 
 // The multi-group launch with delivery at emission.
@@ -675,10 +685,20 @@ int launch_iaf(const IafArgs &A, const SpikeOut &so, const PushOut *po, const Cl
   if (po) {
     launch_k(iaf_push_batch_kernel, g, b, 0, st, A, so, *po, clk, k0, M);
   } else {
-    // small groups in 64-thread blocks, so that they reach every SM (12,500 neurons:
-    // 18.5 -> 18.0 us per 15-step batch)
-    const int tb = n < 148 * 256 ? 64 : 256;
-    launch_k(iaf_batch_kernel, dim3((n + tb - 1) / tb), dim3(tb), 0, st, A, so, clk, k0, M);
+    // Small groups in 64-thread blocks, so that they reach every SM.  Their input two steps ahead
+    // from four steps a batch on: 12,500 neurons, 15 steps, with / without 1.77 / 1.90 us per step of
+    // the network; 5000, 5 steps 2.43 / 2.51; 8000, 3 steps 3.49 / 3.47; 5000, 2 steps 4.88 / 4.77.
+    // Large groups two steps ahead, at the cost of spills, where the batch's accumulators exceed
+    // what stays in L2 and the loads come from memory: 1M neurons, 15 steps (240 MB) 20.5 / 21.8,
+    // 8 steps (128 MB) 21.5 / 21.9, 7 steps (112 MB) 21.8 / 22.0, 5 steps (80 MB) 23.1 / 22.6, one
+    // step 40.1 / 35.2; 300,000, 15 steps (72 MB) 6.65 / 6.55, one step 17.5 / 15.8.
+    const bool small = n < 148 * 256;
+    const bool far = (double)A.in.slot_stride * sizeof(double) * M > 100e6;
+    const int tb = small ? 64 : 256;
+    const dim3 grid((n + tb - 1) / tb);
+    if (small && M >= 4) launch_k(iaf_batch_kernel<64, true>, grid, dim3(tb), 0, st, A, so, clk, k0, M);
+    else if (!small && far) launch_k(iaf_batch_kernel<256, true>, grid, dim3(tb), 0, st, A, so, clk, k0, M);
+    else launch_k(iaf_batch_kernel<256, false>, grid, dim3(tb), 0, st, A, so, clk, k0, M);
   }
   return 1;
 }

@@ -52,3 +52,26 @@ def test_thin_warps_match_oracle(n):
     co, vo = _net(orc.Oracle(), "aeif_cond_beta_multisynapse", n, 10, (0.4, 2.0))
     assert co.sum() > 0 and np.array_equal(c, co)
     assert np.array_equal(v, vo)
+
+
+# group sizes and batch lengths on both sides of the iaf kernel's variants: 64-thread blocks below
+# 37,888 neurons, input two steps ahead there from four steps on, and in large groups where the
+# batch's accumulators exceed 100 MB (15 steps: 416,667 neurons)
+@pytest.mark.parametrize("n,delay", [(1, 0.2), (63, 0.3), (65, 0.4), (37887, 0.3), (37887, 0.4), (37888, 0.4),
+                                     (410000, 1.5), (420000, 1.5)])
+def test_iaf_kernel_variants_match_oracle(n, delay):
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 11)
+        neuron = api.Create("iaf_psc_exp", n)
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 9000.0)
+        api.Connect(pg, neuron, {"rule": "all_to_all"}, {"weight": 60.0, "delay": 1.0, "receptor": 0})
+        api.ConnectFixedIndegreeGPU(neuron, neuron, 2, 40.0, delay, delay, receptor=1, seed=3)
+        api.ActivateSpikeCount(neuron)
+        api.Simulate(9.7)
+        return (np.asarray(api.GetStatus(neuron, "spike_count")).ravel(),
+                np.asarray(api.GetStatus(neuron, "V_m_rel"), dtype=np.float32).ravel())
+    c, v = run(ngpu)
+    co, vo = run(orc.Oracle())
+    assert np.array_equal(c, co) and np.array_equal(v, vo)
+    assert n < 1000 or co.sum() > 0
