@@ -81,8 +81,14 @@ struct Group {
   int2 *d_rec_col = nullptr;
   int *d_pin_off = nullptr;
   PoissonIn *d_pin = nullptr;
-  int *d_pin_tgt = nullptr;      // per poiss_gen edge its target (only if some neuron has several)
-  int pin_lo = 0, pin_hi = 0;    // the edges of neurons lo .. hi-1
+  // where poisson_split holds: the edges drawn by poisson_multi_kernel, their targets, and those of
+  // neurons with one generator that their update kernel draws (null: none)
+  int pin_max = 0;               // generators of the neuron with most of them
+  PoissonIn *d_pin_multi = nullptr;
+  int *d_pin_tgt = nullptr;
+  int n_pin_multi = 0;
+  int *d_pin1_off = nullptr;
+  PoissonIn *d_pin1 = nullptr;
   int *d_sg_off = nullptr, *d_sg_tidx = nullptr, *d_sg_next = nullptr;
   float *d_sg_h = nullptr;
   int lo = 0, hi = 0;            // neurons lo .. hi-1 are simulated by this process (calibration)
@@ -451,10 +457,8 @@ class Engine {
   GroupRecord group_record(Group &g);
   GroupInput group_input(Group &g);
   PoissonMultiArgs poisson_multi_args(Group &g);
-  // the group's poiss_gen draws are made by poisson_multi_kernel, not by its update kernel
-  bool poisson_split(const Group &g) const {
-    return g.d_pin_tgt && !push_ && !(persistent > 0 && persistent_eligible());
-  }
+  int poisson_line(const Group &g) const;
+  bool poisson_split(const Group &g) const;
   void run_steps(long long n);
   void run_batches_partitioned(long long n);
   int part_rank_ = 0, part_world_ = 1;

@@ -386,15 +386,42 @@ void Engine::calibrate() {
       g.d_pin = dalloc<PoissonIn>(pin.size());
       cuda_check(cudaMemcpy(g.d_pin_off, off.data(), (g.n + 1) * sizeof(int), cudaMemcpyHostToDevice), "pin_off");
       cuda_check(cudaMemcpy(g.d_pin, pin.data(), pin.size() * sizeof(PoissonIn), cudaMemcpyHostToDevice), "pin");
-      bool several = false;
-      for (int i = g.lo; i < g.hi; i++) several = several || off[i + 1] - off[i] > 1;
-      if (several) {
-        std::vector<int> tgt(pin.size());
-        for (int i = 0; i < g.n; i++) std::fill(tgt.begin() + off[i], tgt.begin() + off[i + 1], i);
+      for (int i = g.lo; i < g.hi; i++) g.pin_max = std::max(g.pin_max, off[i + 1] - off[i]);
+      if (g.pin_max > 1) {
+        // In large groups with a short update the neurons with one generator keep their draw there;
+        // elsewhere it goes along.  One neuron with a second generator, us per step, one draw kept /
+        // gone along: iaf_psc_exp 1M neurons, 15 steps a batch 20.5 / 24.1, 300,000 6.6 / 7.3; but
+        // 60,000 2.43 / 2.35, 12,500 2.0 / 1.85, and aeif_cond_beta 100,000, 15 steps 11.5 / 10.5.
+        const bool keep = !is_aeif(g.model) && g.hi - g.lo > 148 * 768;
+        std::vector<int> tgt, off1(g.n + 1, 0);
+        std::vector<PoissonIn> multi, single;
+        for (int i = 0; i < g.n; i++) {
+          const int ne = off[i + 1] - off[i];
+          if (ne == 1 && keep) {
+            single.push_back(pin[off[i]]);
+          } else if (i >= g.lo && i < g.hi) {
+            multi.insert(multi.end(), pin.begin() + off[i], pin.begin() + off[i + 1]);
+            tgt.insert(tgt.end(), ne, i);
+          }
+          off1[i + 1] = (int)single.size();
+        }
+        g.n_pin_multi = (int)multi.size();
+        if (single.empty()) {   // every edge in between is one of them
+          g.d_pin_multi = g.d_pin + off[g.lo];
+        } else {
+          g.d_pin_multi = dalloc<PoissonIn>(multi.size());
+          cuda_check(cudaMemcpy(g.d_pin_multi, multi.data(), multi.size() * sizeof(PoissonIn), cudaMemcpyHostToDevice),
+                     "pin");
+        }
         g.d_pin_tgt = dalloc<int>(tgt.size());
         cuda_check(cudaMemcpy(g.d_pin_tgt, tgt.data(), tgt.size() * sizeof(int), cudaMemcpyHostToDevice), "pin");
-        g.pin_lo = off[g.lo];
-        g.pin_hi = off[g.hi];
+        if (!single.empty()) {
+          g.d_pin1_off = dalloc<int>(off1.size());
+          g.d_pin1 = dalloc<PoissonIn>(single.size());
+          cuda_check(cudaMemcpy(g.d_pin1_off, off1.data(), off1.size() * sizeof(int), cudaMemcpyHostToDevice), "pin");
+          cuda_check(cudaMemcpy(g.d_pin1, single.data(), single.size() * sizeof(PoissonIn), cudaMemcpyHostToDevice),
+                     "pin");
+        }
       }
     }
   }
@@ -812,21 +839,50 @@ GroupInput Engine::group_input(Group &g) {
   in.acc = d_acc_ + g.acc_off;
   in.slot_stride = n_acc_;
   if (push_ && g.model == M_IAF_PSC_EXP) in.acc = d_pacc_ + g.acc_off;   // the delivery-at-emission ring
-  in.pin_off = poisson_split(g) ? nullptr : g.d_pin_off;
-  in.pin = g.d_pin;
+  const bool split = poisson_split(g);
+  in.pin_off = split ? g.d_pin1_off : g.d_pin_off;
+  in.pin = split ? g.d_pin1 : g.d_pin;
   in.gen = d_gen_;
   in.lam_scale = (float)(dt / 1000.0);
   in.seed = kernel_seed;
   return in;
 }
 
+// Generators per neuron up to which the draws stay in the update kernel.
+// aeif groups: one.  From two on the update kernel would redo the Philox call and exp(-lambda) of
+// every edge in every step, beside an update that is a latency chain already: 2 generators, 23,000
+// neurons, one / 15 steps a batch 84.6 / 11.5 us per step in the update kernel of an earlier
+// build, 55.4 / 6.9 now.
+// The other updates are short, and the draws' own launch shows where a batch has few steps; nor
+// does one Philox call for four steps help there.  iaf_psc_exp, us per step, own kernel / update
+// kernel, neurons of g generators:
+//   8000, one step: g = 2 9.1 / 7.9, 4 9.0 / 9.1, 6 9.1 / 10.6; two: 2 5.6 / 5.3, 3 5.6 / 5.9; three: 2 4.1 / 4.2
+//   60,000, one step: 4 12.9 / 12.2, 6 14.4 / 15.0; two: 4 8.6 / 8.0, 6 9.8 / 9.7; three: 3 6.0 / 6.0, 4 6.3 / 6.7
+//   1M, one step: 2 55.3 / 46.4, 10 150 / 146; two: 6 80.8 / 73.2, 10 116 / 118; three: 3 42.0 / 42.1, 6 62.2 / 67.4
+//   300,000, six steps: 2 10.9 / 11.0, 4 14.8 / 15.8; 15 steps: 2 9.0 / 9.7, 10 20.9 / 33.1
+// A few such neurons among many hide behind the other warps of a group of several waves: one of
+// 300,000 neurons with 2, six steps, 8.7 / 8.0.
+int Engine::poisson_line(const Group &g) const {
+  if (is_aeif(g.model)) return 1;
+  const int n = g.hi - g.lo;
+  const int size = n < 148 * 256 ? 0 : n <= 148 * 768 ? 1 : 2;
+  static const int line[3][3] = {{4, 2, 1}, {5, 5, 3}, {12, 9, 4}};
+  if (batch_ <= 3) return line[size][batch_ - 1];
+  return size == 2 && 8LL * g.n_pin_multi < n ? 4 : 1;
+}
+
+// Does the group have draws that are made by poisson_multi_kernel, before its update kernel?
+bool Engine::poisson_split(const Group &g) const {
+  return g.pin_max > 1 && g.pin_max > poisson_line(g) && !push_ && !(persistent > 0 && persistent_eligible());
+}
+
 PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
   const GroupInput in = group_input(g);
   PoissonMultiArgs A;
-  A.pin = g.d_pin;
+  A.pin = g.d_pin_multi;
   A.tgt = g.d_pin_tgt;
-  A.e0 = g.pin_lo;
-  A.e1 = g.pin_hi;
+  A.e0 = 0;
+  A.e1 = g.n_pin_multi;
   A.gen = in.gen;
   A.acc = in.acc;
   A.slot_stride = in.slot_stride;
@@ -1222,9 +1278,9 @@ void Engine::set_persistent(int on) {
 // A call costs a table upload, the first step's delivery from the ring and an extra barrier:
 // calls of 1, 2, 4, 8 and 16 steps took 78, 81, 84, 99 and 123 us on the microcircuit at a tenth
 // of its size (79, 85, 92, 110 and 142 us at full size) against 50, 63, 95, 149 and 267 us (54, 72,
-// 109, 184 and 337 us) per batch, so the line lies at four steps.  Neurons with several
-// generators each stay with the per-batch kernels, where poisson_multi_kernel spreads their draws
-// over the GPU.
+// 109, 184 and 337 us) per batch, so the line lies at four steps.  Networks whose draws have a
+// kernel of their own (poisson_split) stay with the per-batch kernels: 8000 neurons of 2 / 4 / 10
+// generators each, loop 4.0 / 5.1 / 9.5 us per step, per batch 7.9 / 9.1 / 9.4.
 // A spiking neuron's edges of total delay one and two steps are delivered by its own block, two
 // warps a spike, while the delivery kernel cuts long segments into parts over the GPU.  us per step,
 // loop / per batch, 20,000 neurons with all delays one step: 1000 edges a source 5.7 / 8.8, 1500
@@ -1238,7 +1294,7 @@ constexpr double LOOP_OWN_EDGES = 2500.0;
 bool Engine::persistent_auto(long long steps) const {
   if (!persistent_eligible() || batch_ != 1 || dmin_ != 0 || steps < LOOP_MIN_STEPS || own_edges_ > LOOP_OWN_EDGES) return false;
   for (auto &g : groups_)
-    if (g.d_pin_tgt) return false;
+    if (poisson_split(g)) return false;
   return true;
 }
 
