@@ -399,8 +399,8 @@ class Engine {
   int *d_strag_cnt_ = nullptr;   // straggler counters, one per aeif group
   int n_strag_ = 0;
   int deliver_blocks_ = 148;
-  int deliver_log2_parts_ = 0;   // delivery: parts per segment, by the mean segment length
-  int deliver_unroll_ = 0;       // delivery: four edges in flight per lane
+  int deliver_long_ = 0;         // delivery: segments in parts, four edges in flight per lane
+  int deliver_log2_parts_ = 0;   // parts per segment, by the mean segment length
   std::map<int, cudaGraphExec_t> graphs_;
   std::vector<void *> allocs_;
   double last_sim_seconds_ = 0.0;

@@ -16,6 +16,7 @@
 #include <cub/block/block_scan.cuh>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ngpu_aeif.cuh"
 #include "ngpu_iaf.cuh"
@@ -440,12 +441,17 @@ __device__ __forceinline__ void reset_stamps(const DeliverArgs &A, long long T, 
 // write weights, and the read-only path asks for data that no one writes during the kernel's life.
 __device__ __forceinline__ uint2 load_edge(const EdgeW *e) { return __ldcg(reinterpret_cast<const uint2 *>(e)); }
 
-// The delivery of one batch by block `block` of `nblocks`; s_pref holds dspan*M+1 ints.
-template <int G, bool AGG = false, bool PF = false>
+// The delivery of one batch; s_pref holds dspan*M+1 ints.  LONG: every segment is cut into
+// 2^log2_parts parts, a work item each, and a lane has four edges in flight; that takes 38 registers
+// instead of 32, six blocks per SM instead of eight, which short segments would pay for nothing.
+// (Both forms in one kernel, 38 registers for all: 1M neurons of 5 edges over 50 delay groups, 10 ms
+// of network 18.9 ms against 13.0 in the short form.)
+template <int G, bool AGG, bool PF, bool LONG>
 __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock *clk, int k0, int M, int *s_pref,
-                                              typename DeliverScan::TempStorage &scan_tmp, int block,
-                                              int nblocks) {
+                                              typename DeliverScan::TempStorage &scan_tmp) {
   typedef DeliverScan Scan;
+  typedef typename std::conditional<LONG, long long, int>::type ItemNo;
+  const int block = blockIdx.x, nblocks = gridDim.x;
   const long long t_first = clk->tidx_base + clk->it0 + k0 + 1;   // time index of step 0
   if (A.stamp) reset_stamps(A, t_first, block, nblocks);
   const int npairs = A.dspan * M;
@@ -496,10 +502,10 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
     float height;
     long long e0, e1;
   };
-  // (long segments are cut: the parts of a segment are consecutive work items)
-  const int lp = A.log2_parts;
-  const long long total_parts = (long long)total << lp;
-  auto fetch = [&](long long item_part) {
+  // (the parts of a segment are consecutive work items)
+  const int lp = LONG ? A.log2_parts : 0;
+  const ItemNo total_parts = (ItemNo)total << lp;
+  auto fetch = [&](ItemNo item_part) {
     const int item = (int)(item_part >> lp), part = (int)(item_part & ((1 << lp) - 1));
     int lo = 0, hi = npairs;   // pair with s_pref[pr] <= item < s_pref[pr+1]
     while (hi - lo > 1) {
@@ -517,7 +523,7 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
     it.height = __int_as_float(sp.y);
     it.e0 = __ldg(&A.ev_off[key]);
     it.e1 = __ldg(&A.ev_off[key + 1]);
-    if (lp) {
+    if constexpr (LONG) {
       const long long c = (it.e1 - it.e0 + (1 << lp) - 1) >> lp;
       it.e0 = min(it.e1, it.e0 + part * c);
       it.e1 = min(it.e1, it.e0 + c);
@@ -553,9 +559,9 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
         if (valid && lane == __ffs(peers) - 1) atomicAdd(&acc[ew.x], v);
       }
     } else {
-      const EdgeW *edge = A.edge + e0;
-      const int len = (int)(e1 - e0);
-      if (A.unroll) {          // four loads in flight per lane before their reductions
+      if constexpr (LONG) {          // four loads in flight per lane before their reductions
+        const EdgeW *edge = A.edge + e0;
+        const int len = (int)(e1 - e0);
         for (int e = sub; e < len; e += 4 * G) {
           uint2 ew[4];
 #pragma unroll
@@ -566,8 +572,10 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
             if (e + u * G < len) atomicAdd(&acc[ew[u].x], (double)__fmul_rn(height, __uint_as_float(ew[u].y)));
         }
       } else {
-        for (int e = sub; e < len; e += G) {
-          const uint2 ew = load_edge(edge + e);
+        // (not unrolled: the compiler's four turns at once take 60 registers)
+#pragma unroll 1
+        for (long long e = e0 + sub; e < e1; e += G) {
+          const uint2 ew = load_edge(A.edge + e);
           atomicAdd(&acc[ew.x], (double)__fmul_rn(height, __uint_as_float(ew.y)));
         }
       }
@@ -577,11 +585,11 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
   if constexpr (PF) {
     // software pipeline: the next item's ring entry and segment offsets are loaded before
     // this item's edges, so their dependent latencies overlap this item's traffic
-    long long item = grp;
+    ItemNo item = grp;
     Item cur;
     if (item < total_parts) cur = fetch(item);
     while (item < total_parts) {
-      const long long next = item + ngrp;
+      const ItemNo next = item + ngrp;
       Item nxt;
       if (next < total_parts) nxt = fetch(next);
       deliver(cur);
@@ -589,7 +597,7 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
       item = next;
     }
   } else {
-    for (long long item = grp; item < total_parts; item += ngrp) deliver(fetch(item));
+    for (ItemNo item = grp; item < total_parts; item += ngrp) deliver(fetch(item));
   }
   // one counter update per block
   for (int o = 16; o > 0; o >>= 1) nev += __shfl_down_sync(0xffffffffu, nev, o);
@@ -602,13 +610,13 @@ __device__ __forceinline__ void deliver_batch(const DeliverArgs &A, const Clock 
   __syncthreads();
 }
 
-template <int G, bool AGG = false, bool PF = false>
+template <int G, bool AGG, bool PF, bool LONG>
 __global__ void __launch_bounds__(DELIVER_THREADS) deliver_batch_kernel(const DeliverArgs A,
                                                                         const Clock *clk, int k0, int M) {
   pdl_enter();
   extern __shared__ int s_pref[];   // npairs + 1 prefix sums over (delay group, arrival step)
   __shared__ typename DeliverScan::TempStorage scan_tmp;
-  deliver_batch<G, AGG, PF>(A, clk, k0, M, s_pref, scan_tmp, blockIdx.x, gridDim.x);
+  deliver_batch<G, AGG, PF, LONG>(A, clk, k0, M, s_pref, scan_tmp);
 }
 
 __global__ void clock_advance_kernel(Clock *clk, int K) {
@@ -730,20 +738,31 @@ int launch_spike_gen(const SpikeGenArgs &A, const SpikeOut &so, const Clock *clk
   return 1;
 }
 
+template <int G, bool PF>
+static void launch_deliver_g(const DeliverArgs &A, dim3 g, size_t smem, const Clock *clk, int k0, int M, cudaStream_t st) {
+  const dim3 b(DELIVER_THREADS);
+  if constexpr (G == 32) {
+    if (A.aggregate) {
+      launch_k(deliver_batch_kernel<32, true, PF, false>, g, b, smem, st, A, clk, k0, M);
+      return;
+    }
+  }
+  if (A.long_segments) launch_k(deliver_batch_kernel<G, false, PF, true>, g, b, smem, st, A, clk, k0, M);
+  else launch_k(deliver_batch_kernel<G, false, PF, false>, g, b, smem, st, A, clk, k0, M);
+}
+
 int launch_deliver(const DeliverArgs &A, int n_blocks, int group, const Clock *clk, int k0, int M,
                    cudaStream_t st) {
   const size_t smem = (size_t)(A.dspan * M + 1) * sizeof(int);
-  const dim3 g(n_blocks), b(DELIVER_THREADS);
+  const dim3 g(n_blocks);
   if (A.prefetch) {
-    if (group == 8) launch_k(deliver_batch_kernel<8, false, true>, g, b, smem, st, A, clk, k0, M);
-    else if (group == 16) launch_k(deliver_batch_kernel<16, false, true>, g, b, smem, st, A, clk, k0, M);
-    else if (A.aggregate) launch_k(deliver_batch_kernel<32, true, true>, g, b, smem, st, A, clk, k0, M);
-    else launch_k(deliver_batch_kernel<32, false, true>, g, b, smem, st, A, clk, k0, M);
+    if (group == 8) launch_deliver_g<8, true>(A, g, smem, clk, k0, M, st);
+    else if (group == 16) launch_deliver_g<16, true>(A, g, smem, clk, k0, M, st);
+    else launch_deliver_g<32, true>(A, g, smem, clk, k0, M, st);
   } else {
-    if (group == 8) launch_k(deliver_batch_kernel<8>, g, b, smem, st, A, clk, k0, M);
-    else if (group == 16) launch_k(deliver_batch_kernel<16>, g, b, smem, st, A, clk, k0, M);
-    else if (A.aggregate) launch_k(deliver_batch_kernel<32, true>, g, b, smem, st, A, clk, k0, M);
-    else launch_k(deliver_batch_kernel<32>, g, b, smem, st, A, clk, k0, M);
+    if (group == 8) launch_deliver_g<8, false>(A, g, smem, clk, k0, M, st);
+    else if (group == 16) launch_deliver_g<16, false>(A, g, smem, clk, k0, M, st);
+    else launch_deliver_g<32, false>(A, g, smem, clk, k0, M, st);
   }
   return 1;
 }

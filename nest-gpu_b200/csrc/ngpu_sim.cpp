@@ -488,23 +488,29 @@ void Engine::calibrate() {
   d_clk_ = dalloc<Clock>(1);
   cuda_check(cudaMemset(d_clk_, 0, sizeof(Clock)), "clock");
   deliver_blocks_ = std::max(1, std::min(148 * 8, (n_src_out + 63) / 64));
+  const double mean_len = n_src_out > 0 ? (double)n_edge_dev_ / ((double)n_src_out * dspan_) : 0.0;
   // With slots of many megabytes fewer work items in flight keep fewer arrival steps open, so that
   // the reductions stay in L2.  Blocks 296 / 592 / 1184, ms: 500k AdEx (8 MB a slot, 30 ms) 12.0 /
   // 11.0 / 11.1, 1M (16 MB, 50 ms) 34.6 / 31.8 / 34.7, 2.8M ensemble (45 MB, 20 ms) 24.6 / 26.9 /
-  // 28.4; 250k and less take all the blocks there are.
-  while (deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184) deliver_blocks_ /= 2;
+  // 28.4; 250k and less take all the blocks there are.  Short segments, chains of dependent loads
+  // for a few reductions, need all of them: 1M iaf_psc_exp neurons, 592 / 1184, ms per 10 ms,
+  // segments of 200 edges 3.49 / 3.88, 90 edges 7.46 / 8.22, 9 edges 4.55 / 3.86, one edge or none
+  // 21.6 / 13.0; and short batches have few arrival steps anyway (100 edges, one step 4.08 / 3.88).
+  while (mean_len >= 32.0 && batch_ >= 8 && deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184)
+    deliver_blocks_ /= 2;
   // Long (source, delay) segments are delivered in parts of about 128 edges (the four loads that a
   // 32-lane group has in flight), so that a batch's few spikes fill the GPU: 12,500 neurons with
-  // 1250 edges per segment, 500 spikes a batch, 25.9 -> 12.3 us.  Networks with large accumulator
-  // slots have spikes enough, and more edges in flight only widen the set of addresses that L2 has
-  // to hold: parts and four loads per lane took 209 instead of 175 us on the 1M network (16 MB a
-  // slot) and 727 instead of 644 us on the 2.8M ensemble (45 MB).
-  deliver_unroll_ = (double)n_acc_ * sizeof(double) <= 12e6 ? 1 : 0;
+  // 1250 edges per segment, 500 spikes a batch, 25.9 -> 12.3 us.  Networks whose batch has large
+  // accumulators have spikes enough, and more edges in flight only widen the set of addresses that
+  // L2 has to hold.  In parts / whole, us per 10 ms, by the accumulators of the batch and the mean
+  // segment: 0.6 MB, 100 edges 1075 / 1168; 3 MB, 1250 324 / 372; 4.8 MB, 300 1980 / 2341; 6.4 MB,
+  // 166 411 / 430; but 16 MB, 67 474 / 441; 24 MB, 64 231 / 219 and 300 1133 / 1075; 32 MB, 90 1539 /
+  // 1499; 144 MB, 300 2576 / 2483.  By length: 0.1 MB, 64 edges 144 / 148; 0.5 MB, 42 edges 206 / 212;
+  // but 0.3 MB, 18 edges 236 / 229; 1 MB, 7 edges 1537 / 1321.
+  deliver_long_ = mean_len >= 32.0 && (double)n_acc_ * sizeof(double) * batch_ <= 12e6;
   deliver_log2_parts_ = 0;
-  if (n_src_out > 0 && deliver_unroll_) {
-    const double mean_len = (double)n_edge_dev_ / ((double)n_src_out * dspan_);
+  if (deliver_long_)
     while (deliver_log2_parts_ < 4 && mean_len > (128 << deliver_log2_parts_)) deliver_log2_parts_++;
-  }
   if (plastic_) build_plastic(pl_edge, pl_key, pl_rank);
   // ---- dendritic delays: the reverse ring (plastic networks only; src/spike_buffer.cu:162-317)
   if (plastic_) {
@@ -1040,8 +1046,8 @@ DeliverArgs Engine::deliver_args() {
   A.n_events = d_counters_ + 1;
   A.strag_cnt = d_strag_cnt_;
   A.n_strag = n_strag_;
+  A.long_segments = deliver_long_;
   A.log2_parts = deliver_log2_parts_;
-  A.unroll = deliver_unroll_;
   A.aggregate = deliver_aggregate;
   A.prefetch = deliver_prefetch;
   A.xch = part_world_ > 1 ? xch_send_ : nullptr;

@@ -267,8 +267,8 @@ struct DeliverArgs {
   unsigned long long *n_events;
   int *strag_cnt;        // per-group straggler counters, cleared for the batch
   int n_strag;
-  int log2_parts;        // every segment is delivered in 2^log2_parts parts, a work group each
-  int unroll;            // 1: four edges in flight per lane
+  int long_segments;     // 1: every segment is delivered in 2^log2_parts parts, a work group each, with
+  int log2_parts;        // four edges in flight per lane
   int aggregate;         // 1 (with 32-lane groups): warp-aggregated reductions
   int prefetch;          // 1: the next work item's ring entry and offsets loaded ahead
   int4 *xch;             // partitioned network: exchange buffer whose count the batch clears

@@ -75,3 +75,28 @@ def test_iaf_kernel_variants_match_oracle(n, delay):
     co, vo = run(orc.Oracle())
     assert np.array_equal(c, co) and np.array_equal(v, vo)
     assert n < 1000 or co.sum() > 0
+
+
+# both forms of the delivery kernel (parts and four edges in flight from 32 edges a segment on, while
+# the batch's accumulators stay below 12 MB; whole segments otherwise) and every lane group
+@pytest.mark.parametrize("n,k,hi", [(64, 31, 1.5), (64, 33, 1.5), (200, 40, 4.0), (52000, 33, 1.5)])
+@pytest.mark.parametrize("group,prefetch", [(32, False), (16, True), (8, False)])
+def test_delivery_forms_match_oracle(n, k, hi, group, prefetch):
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 5)
+        neuron = api.Create("iaf_psc_exp", n)
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 8000.0)
+        api.Connect(pg, neuron, {"rule": "all_to_all"}, {"weight": 45.0, "delay": 1.0, "receptor": 0})
+        api.ConnectFixedIndegreeGPU(neuron, neuron, k, 100.0 / k, 1.5, hi, receptor=0, seed=3)
+        api.ActivateSpikeCount(neuron)
+        api.Simulate(14.3)
+        return (np.asarray(api.GetStatus(neuron, "spike_count")).ravel(),
+                np.asarray(api.GetStatus(neuron, "V_m_rel"), dtype=np.float32).ravel())
+    ngpu.SetDeliverGroup(group)
+    ngpu.SetDeliverPrefetch(prefetch)
+    c, v = run(ngpu)
+    o = orc.Oracle()
+    co, vo = run(o)
+    assert co.sum() > 0 and np.array_equal(c, co) and np.array_equal(v, vo)
+    assert ngpu.GetStats()["n_events"] == o.NEvents()
