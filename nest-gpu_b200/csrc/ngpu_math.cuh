@@ -20,14 +20,15 @@
 
 namespace ngpu {
 
-// Correctly rounded 1 / b for normal b below 2^126 without a branch, so that several pipeline (the
+// Correctly rounded 1 / b for b in [1/16, 2^126) without a branch, so that several pipeline (the
 // compiler's division and __frcp_rn each carry a branch to a slow path: the six of an RK5 step
 // were a serial chain of 430 of the step's 1900 cycles).  One Newton step with fused multiply-adds
 // from the hardware approximation: Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34 (1990), shows it correctly rounded from an
 // approximation within one ulp unless the significand of b is all ones, where the quotient lies
 // just above a power of two and the approximation is already the result.  The test compares it
-// with __frcp_rn over every float in range.
+// with __frcp_rn over every float of that range, which covers its callers: error scales (0.1 and
+// above), fourth roots of errors above 1, and m + 1 of log_m.
 __device__ __forceinline__ float rcp_m(float b) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));

@@ -64,30 +64,37 @@ double measure_random_reduction_rate(size_t bytes, long long n_ops) {
 // The branch-free reciprocal and quotient of ngpu_math.cuh against the compiler's correctly
 // rounded ones: every float from 1/16 up to 2^126, and every quotient that log_m forms.
 // ---------------------------------------------------------------------------
-__global__ void check_rounded_kernel(unsigned long long *bad) {
+constexpr unsigned RCP_FIRST = 0x3d800000u, RCP_END = 0x7e800000u;   // 1/16, 2^126
+constexpr unsigned LOG_FIRST = 0x3f3504f0u, LOG_LAST = 0x3fb504f8u;  // sqrt(1/2) .. sqrt(2)
+
+// n[0]: inputs on which they differ; n[1]: inputs compared
+__global__ void check_rounded_kernel(unsigned long long *n_out) {
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   const unsigned long long i0 = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-  unsigned long long n = 0;
-  for (unsigned long long b = 0x3d800000ull + i0; b < 0x7e800000ull; b += stride) {
+  unsigned long long n = 0, seen = 0;
+  for (unsigned long long b = RCP_FIRST + i0; b < RCP_END; b += stride, seen++) {
     const float x = __uint_as_float((unsigned)b);
     n += __float_as_uint(rcp_m(x)) != __float_as_uint(__frcp_rn(x));
   }
-  for (unsigned long long b = 0x3f3504f0ull + i0; b <= 0x3fb504f8ull; b += stride) {   // sqrt(1/2) .. sqrt(2)
+  for (unsigned long long b = LOG_FIRST + i0; b <= LOG_LAST; b += stride, seen++) {
     const float m = __uint_as_float((unsigned)b), num = __fsub_rn(m, 1.0f), den = __fadd_rn(m, 1.0f);
     n += __float_as_uint(div_m(num, den)) != __float_as_uint(__fdiv_rn(num, den));
   }
-  if (n) atomicAdd(bad, n);
+  if (n) atomicAdd(n_out, n);
+  atomicAdd(n_out + 1, seen);
 }
 
-// Number of inputs on which they differ (-1: the check could not run).
+// Number of inputs on which they differ (-1: not all of them were compared).
 long long check_rounded_ops() {
-  unsigned long long *d = nullptr, h = 0;
+  unsigned long long *d = nullptr, h[2] = {0, 0};
   if (cudaMalloc(&d, sizeof(h)) != cudaSuccess) return -1;
-  cudaMemset(d, 0, sizeof(h));
+  bool ok = cudaMemset(d, 0, sizeof(h)) == cudaSuccess;
   check_rounded_kernel<<<148 * 8, 256>>>(d);
-  const bool ok = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess;
+  ok = cudaGetLastError() == cudaSuccess && ok;
+  ok = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess && ok;
   cudaFree(d);
-  return ok ? (long long)h : -1;
+  const unsigned long long want = (unsigned long long)(RCP_END - RCP_FIRST) + (LOG_LAST - LOG_FIRST + 1);
+  return ok && h[1] == want ? (long long)h[0] : -1;
 }
 
 }  // namespace ngpu
