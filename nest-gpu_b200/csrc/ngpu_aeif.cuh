@@ -492,6 +492,16 @@ __device__ __forceinline__ void rk5_begin(const float *y, float h, const AeifQ<M
   constexpr int NVM = 2 + AeifShape<MODEL>::npv * PMAX;
   const int NV = 2 + AeifShape<MODEL>::npv * q.ports();
   aeif_derivs(y, k1, q, refr);
+  if constexpr (!FIXED) {   // run-time port count: the arrays live in local memory, one pass over them
+#pragma unroll
+    for (int i = 0; i < NVM; i++) {
+      if (i < NV) {
+        const float ys = __fadd_rn(__fadd_rn(fabsf(y[i]), fabsf(__fmul_rn(k1[i], h))), ck::scal_min);
+        iys[i] = __fdiv_rn(1.0f, ys);
+      }
+    }
+    return;
+  }
   bool normal = true;
 #pragma unroll
   for (int i = 0; i < NVM; i++) {
@@ -558,11 +568,13 @@ __device__ __forceinline__ float rk5_trial(const float *y, float &h, float hmin,
   const float f1 = __fmul_rn(h, ck::e1), f3 = __fmul_rn(h, ck::e3), f4 = __fmul_rn(h, ck::e4),
               f5 = __fmul_rn(h, ck::e5), f6 = __fmul_rn(h, ck::e6);
   // error terms two variables at a time (lane-exact, as in stage_comb)
-  float e[NVM];
+  float e[FIXED ? NVM : 1], err = 0.0f;
 #pragma unroll
   for (int i = 0; i < NVM; i += (FIXED ? 2 : 1)) {
-    e[i] = 0.0f;
-    if (FIXED && i + 1 < NVM) e[i + 1] = 0.0f;
+    if constexpr (FIXED) {
+      e[i] = 0.0f;
+      if (i + 1 < NVM) e[i + 1] = 0.0f;
+    }
     if (i < NV) {
       if (FIXED && i + 1 < NVM) {
         float2 v = __fmul2_rn(make_float2(f1, f1), make_float2(k1[i], k1[i + 1]));
@@ -576,11 +588,12 @@ __device__ __forceinline__ float rk5_trial(const float *y, float &h, float hmin,
       } else {
         float v = __fmaf_rn(f6, k6[i], __fmaf_rn(f5, k5[i], __fmaf_rn(f4, k4[i],
                                                                       __fmaf_rn(f3, k3[i], __fmul_rn(f1, k1[i])))));
-        e[i] = __fmul_rn(v, iys[i]);
+        v = __fmul_rn(v, iys[i]);
+        if constexpr (FIXED) e[i] = v;
+        else err = (err > fabsf(v)) ? err : fabsf(v);
       }
     }
   }
-  float err = 0.0f;
   if constexpr (FIXED) {
     err = max_abs<NVM>(e);
     if (err != err) {     // the reference's scan forgets a NaN that a later variable follows
@@ -589,25 +602,29 @@ __device__ __forceinline__ float rk5_trial(const float *y, float &h, float hmin,
       for (int i = 0; i < NVM; i++)
         if (i < NV) err = (err > fabsf(e[i])) ? err : fabsf(e[i]);
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < NVM; i++)
-      if (i < NV) err = (err > fabsf(e[i])) ? err : fabsf(e[i]);
   }
   return __fmul_rn(err, ck::inv_eps);
 }
 
 // Step size of the next trial after a rejection: max(0.9 h err^-1/4, 0.1 h).
+template <bool FIXED>
 __device__ __forceinline__ float rk5_shrink(float h, float err) {
   const float r4 = __fsqrt_rn(__fsqrt_rn(err));   // err > 1, or NaN
-  float hnew = __fmul_rn(__fmul_rn(h, ck::coeff), r4 < RCP_MAX ? rcp_m(r4) : __fdiv_rn(1.0f, r4));
+  float hnew = __fmul_rn(__fmul_rn(h, ck::coeff), FIXED && r4 < RCP_MAX ? rcp_m(r4) : __fdiv_rn(1.0f, r4));
   float h01 = __fmul_rn(0.1f, h);
   return (hnew > h01) ? hnew : h01;
 }
 
 // Step size proposed after an accepted trial: 0.9 h err^-1/5, or 5 h for a tiny error.  Both are
-// computed (no branch), so that the caller's next instructions overlap the chain of log and exp.
+// computed (no branch), so that the caller's next instructions overlap the chain of log and exp;
+// not in the kernel for any number of ports, which is bound by its spills.
+template <bool FIXED>
 __device__ __forceinline__ float rk5_grow(float h, float err, float hmin) {
+  if constexpr (!FIXED) {
+    if (err > ck::err_min) h = __fmul_rn(__fmul_rn(h, ck::coeff), exp_m(__fmul_rn(-0.2f, log_m<false>(err))));
+    else h = __fmul_rn(5.0f, h);
+    return (h == h) ? h : hmin;
+  }
   const float hl = __fmul_rn(__fmul_rn(h, ck::coeff), exp_m(__fmul_rn(-0.2f, log_m(err))));
   h = (err > ck::err_min) ? hl : __fmul_rn(5.0f, h);
   return (h == h) ? h : hmin;
@@ -620,7 +637,7 @@ struct StepCtl {
   float err = 0.0f;
   bool grow = false;      // h is the last trial's and still to be grown
   __device__ __forceinline__ void settle(float &h, float hmin) {
-    const float hg = rk5_grow(h, err, hmin);
+    const float hg = rk5_grow<true>(h, err, hmin);
     h = grow ? hg : h;
     grow = false;
   }
@@ -681,7 +698,7 @@ __device__ __forceinline__ int rk5_step(double &x, float *y, float &h, float hmi
       atomicOr(status, ST_RK5_TRIALS);
       break;
     }
-    h = rk5_shrink(h, err);
+    h = rk5_shrink<FIXED>(h, err);
   }
   if (LM == LM_LOG) {
     const unsigned long long pos = atomicAdd(L.log_cursor, 1ULL);
@@ -694,7 +711,7 @@ __device__ __forceinline__ int rk5_step(double &x, float *y, float &h, float hmi
     }
   }
   x += (double)h;
-  h = rk5_grow(h, err, hmin);
+  h = rk5_grow<FIXED>(h, err, hmin);
 #pragma unroll
   for (int i = 0; i < NVM; i++)
     if (i < NV) y[i] = yn[i];
@@ -717,7 +734,7 @@ __device__ __forceinline__ bool aeif_substep(const AeifArgs &A, const SpikeOut &
                                              unsigned long long &nd, const float *smodel, int &guard) {
   const double x1 = tnow;
   const float hmax = (float)(x1 - x);
-  if constexpr (LM == LM_PLAIN) {
+  if constexpr (LM == LM_PLAIN && FIXED) {
     constexpr int NVM = 2 + AeifShape<MODEL>::npv * PMAX;
     const int NV = 2 + AeifShape<MODEL>::npv * q.ports();
     float k1[NVM], yn[NVM], iys[NVM];
@@ -732,7 +749,7 @@ __device__ __forceinline__ bool aeif_substep(const AeifArgs &A, const SpikeOut &
         atomicOr(so.status, ST_RK5_TRIALS);
         break;
       }
-      h = rk5_shrink(h, ctl.err);
+      h = rk5_shrink<FIXED>(h, ctl.err);
     }
     x += (double)h;
     ctl.grow = true;
@@ -756,8 +773,10 @@ __device__ __forceinline__ bool aeif_external(const AeifArgs &A, const SpikeOut 
   const double x1 = tnow;
   const bool end = (x >= x1 - (double)A.hmin);
   ++guard;
-  const bool rare = guard > ck::max_substeps || y[0] < -1.0e3f || fabsf(y[1]) > 1.0e6f || refr > 0.0f || y[0] >= q.V_peak;
-  if (!rare) return end;
+  if constexpr (FIXED) {
+    const bool rare = guard > ck::max_substeps || y[0] < -1.0e3f || fabsf(y[1]) > 1.0e6f || refr > 0.0f || y[0] >= q.V_peak;
+    if (!rare) return end;
+  }
   if (guard > ck::max_substeps) {
     atomicOr(so.status, ST_RK5_TRIALS);
     return true;
@@ -882,7 +901,7 @@ __device__ __forceinline__ bool aeif_tpi_iter(const AeifArgs &A, const SpikeOut 
   nd += 5;
   if (!(err <= 1.0f || h <= A.hmin_acc)) {
     if (++trials < ck::max_trials) {
-      h = rk5_shrink(h, err);
+      h = rk5_shrink<FIXED>(h, err);
       return false;
     }
     atomicOr(so.status, ST_RK5_TRIALS);
@@ -912,8 +931,12 @@ __device__ __forceinline__ bool aeif_tpi_iter(const AeifArgs &A, const SpikeOut 
 // step stay in registers across iterations; a lane is handed to the straggler kernel
 // only between accepted steps, so every lane runs the same sequence of operations as
 // in the step-at-once form and results are identical.
+// One port with uniform parameters, OCC = 0: capped at 128 registers, eight 64-thread blocks per SM.
+// The step's controller state took it from 124 to 134, seven blocks, and 150,000 quiet psc_exp
+// neurons in one-step batches from 16.1 to 18.0 us per step; 118 to 120 registers with the cap, no
+// spills.
 template <int MODEL, int PMAX, bool FIXED, int LM, int OCC = 0, bool UNI = false, bool TPI = false>
-__global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2 ? 5 : 1))
+__global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2 ? 5 : (PMAX == 1 && UNI ? 2 : 1)))
     aeif_batch_kernel(const AeifArgs A, const SpikeOut so,
                                                          const Clock *clk, int k0, int M) {
   pdl_enter();
@@ -986,7 +1009,7 @@ __global__ void __launch_bounds__(OCC == 2 ? 128 : 256, OCC == 1 ? 3 : (OCC == 2
         }
       }
     }
-    if (LM == LM_PLAIN) ctl.settle(h, A.hmin);
+    if (LM == LM_PLAIN && FIXED) ctl.settle(h, A.hmin);
     aeif_store<MODEL, PMAX, FIXED>(A, i, y, refr, x, h, NV);
     if (deferred) {
       const int pos = atomicAdd(A.strag_cnt, 1);
@@ -1044,7 +1067,7 @@ __global__ void __launch_bounds__(128, 1) aeif_straggler_kernel(const AeifArgs A
         }
       }
     }
-    if (LM == LM_PLAIN) ctl.settle(h, A.hmin);
+    if (LM == LM_PLAIN && FIXED) ctl.settle(h, A.hmin);
     aeif_store<MODEL, PMAX, FIXED>(A, i, y, refr, x, h, NV);
   }
   warp_add(A.nderiv, nd);

@@ -911,11 +911,19 @@ PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
 // neuron parameters) 60k 2.88 / 3.68, 100k 3.58 / 4.00, 300k 7.75 / 6.45.  128-thread blocks are
 // the same or slower.  One-step batches pay the second launch every step: 80k 20.2 / 22.7, 180k
 // 25.4 / 25.7, so there the line lies at three waves.
+// Five ports and more run in one kernel for any number of them, whose state lies in local memory.
+// There a batch's stragglers are worth a hand-off at every size, and a thin warp's loads fill a line
+// each: 128-thread blocks of full warps, hand-off after M + 4.  beta with 6 ports, us per 10 ms, so /
+// by the rules for fewer ports: 1000 neurons 2086 / 5342 (quiet), 11,010 / 11,302 (active), 30,000
+// 20,567 / 28,174.  The same for one port in one-step batches beyond the resident neurons: 150,000
+// active beta neurons 9.1 ms per 10 ms, 13.1 without a hand-off (quiet 1.34, 1.46).
 void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
-  const bool hand_off = A.hi - A.lo > (batch_ == 1 ? 3 * g.resident : g.resident);
-  const int budget = rk5_budget >= 0 ? rk5_budget : (hand_off ? 1 : 0);
+  const bool any_ports = g.nport > 4;
+  const bool late = any_ports || (g.nport == 1 && batch_ == 1 && A.hi - A.lo > g.resident);
+  const bool hand_off = !late && A.hi - A.lo > (batch_ == 1 ? 3 * g.resident : g.resident);
+  const int budget = rk5_budget >= 0 ? rk5_budget : late ? 4 : (hand_off ? 1 : 0);
   A.budget = budget > 0 ? batch_ + budget : 0;
-  A.threads = update_threads > 0 ? update_threads : 64;
+  A.threads = update_threads > 0 ? update_threads : late ? 128 : 64;
   A.occupancy = update_occupancy >= 0 ? update_occupancy : (hand_off ? 2 : 0);
   A.trial_iter = update_trial_iter >= 0 ? update_trial_iter : (hand_off ? 1 : 0);
   // The lanes of a warp wait for each other in every step (rejected trials, the network's
@@ -924,7 +932,7 @@ void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
   // per warp), with the step model 327 / 261; but 23k neurons 81 / 88.6 at 16 per warp (ten warps
   // per SM) and 6000 55.9 / 56.5 at four: more warps than that slow each other down.
   A.log2_lanes = 5;
-  while (A.log2_lanes > 0 && (A.hi - A.lo) <= (148LL * 7 << (A.log2_lanes - 1))) A.log2_lanes--;
+  while (!any_ports && A.log2_lanes > 0 && (A.hi - A.lo) <= (148LL * 7 << (A.log2_lanes - 1))) A.log2_lanes--;
 }
 
 Engine::Mapping Engine::mapping_in_use() const {

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import nestgpu as ngpu
+import oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -119,3 +120,29 @@ def test_long_first_segments_stay_with_the_per_batch_kernels(k, hi, loop):
     assert got[1].sum() > 0
     for other in (off, on):
         assert np.array_equal(got[1], other[1]) and np.array_equal(got[2], other[2])
+
+
+@pytest.mark.parametrize("ports,n,delay,want", [(5, 60, 1.0, (128, 0, 0, 4)), (20, 33, 0.3, (128, 0, 0, 4)),
+                                                (1, 60, 0.1, (64, 0, 0, 0)), (1, 130000, 0.1, (128, 0, 0, 4))])
+def test_one_port_and_any_number_of_ports(ports, n, delay, want):
+    """The mappings of their own, against the oracle where that is quick."""
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 4)
+        neuron = api.Create("aeif_cond_beta_multisynapse", n, ports)
+        api.SetStatus(neuron, {"E_rev": [-85.0 if p % 3 == 2 else 0.0 for p in range(ports)],
+                               "tau_decay": [2.0 + p for p in range(ports)], "tau_rise": [1.0 + 0.5 * p for p in range(ports)]})
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 8000.0)
+        api.Connect(pg, neuron, {"rule": "all_to_all"}, {"weight": 1.0, "delay": 1.0, "receptor": 0})
+        for p in range(ports):
+            api.ConnectFixedIndegreeGPU(neuron, neuron, 3, 0.2, delay, delay, receptor=p, seed=p + 1)
+        api.ActivateSpikeCount(neuron)
+        api.Simulate(20.0 if n < 1000 else 1.0)
+        return (np.asarray(api.GetStatus(neuron, "spike_count")).ravel(),
+                np.asarray(api.GetStatus(neuron, "V_m"), dtype=np.float32).ravel())
+    c, v = run(ngpu)
+    m = ngpu.GetLaunchMapping()
+    assert (m["update_threads"], m["update_occupancy"], m["update_trial_iter"], m["rk5_budget"]) == want
+    if n < 1000:
+        co, vo = run(orc.Oracle())
+        assert co.sum() > 0 and np.array_equal(c, co) and np.array_equal(v, vo)
