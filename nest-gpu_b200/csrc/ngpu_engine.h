@@ -426,6 +426,8 @@ class Engine {
   IafArgs *d_iaf_tab_ = nullptr;
   int *d_iaf_blk0_ = nullptr;
   int *d_iaf_first_ = nullptr;   // neuron prefix over the iaf groups
+  bool iaf_tab_valid_ = false;   // d_iaf_tab_ holds the present arguments (until invalidate_graphs)
+  unsigned long long iaf_tab_seed_ = 0;
   GridBarrier *d_bar_ = nullptr;
   volatile long long *h_skipped_ = nullptr;   // steps that persistent launches left out (pinned, device-visible)
   bool loop_failed_ = false;     // a launch was refused or timed out: per batch until SetPersistent

@@ -84,6 +84,7 @@ void Engine::free_device() {
 }
 
 void Engine::invalidate_graphs() {
+  iaf_tab_valid_ = false;
   for (auto &kv : graphs_) cudaGraphExecDestroy(kv.second);
   graphs_.clear();
 }
@@ -442,19 +443,13 @@ void Engine::calibrate() {
       if (g.model == M_IAF_PSC_EXP) n_iaf += g.n;
     pers_blocks_ = persistent_blocks(n_iaf, dspan_);
   }
-  if (pers_blocks_) {
-    void *p = nullptr;
-    cuda_check(cudaHostAlloc(&p, sizeof(long long), cudaHostAllocMapped), "pinned counter");
-    h_skipped_ = (volatile long long *)p;
-    *h_skipped_ = 0;
-    own_edges_ = 0.0;
-    if (dmin_ == 0 && n_src_out > 0) {
-      unsigned long long *d_sum = dalloc<unsigned long long>(1);
-      cuda_check(cudaMemset(d_sum, 0, sizeof(*d_sum)), "memset");
-      const long long sum = persistent_own_edges(d_ev_off_, N, dspan_, d_sum);
-      if (sum < 0) throw NgpuError("counting the edges of the first delays failed");
-      own_edges_ = (double)sum / n_src_out;
-    }
+  own_edges_ = 0.0;
+  if (pers_blocks_ && dmin_ == 0 && n_src_out > 0) {
+    unsigned long long *d_sum = dalloc<unsigned long long>(1);
+    cuda_check(cudaMemset(d_sum, 0, sizeof(*d_sum)), "memset");
+    const long long sum = persistent_own_edges(d_ev_off_, N, dspan_, d_sum);
+    if (sum < 0) throw NgpuError("counting the edges of the first delays failed");
+    own_edges_ = (double)sum / n_src_out;
   }
   const size_t acc_slots = pers_blocks_ ? std::max(batch_, 4) : batch_;
   d_acc_ = dalloc<double>(n_acc_ * acc_slots);
@@ -1246,9 +1241,11 @@ void Engine::launch_batch(int k0, int M, std::vector<cudaEvent_t> *ev) {
   set_launch_pdl(false);
 }
 
-// Argument table of the iaf groups for the single multi-group launch; rebuilt before
-// each graph capture (the arguments hold record-buffer pointers that can change).
+// Argument table of the iaf groups for the single multi-group launch and the persistent loop;
+// rebuilt when the arguments, which captured graphs hold too, have changed (a build waits for the
+// stream and copies three times, 25 us).
 void Engine::prepare_multi() {
+  if (iaf_tab_valid_ && iaf_tab_seed_ == kernel_seed) return;
   std::vector<IafArgs> tab;
   std::vector<int> blk0, first{0};
   int nb = 0;
@@ -1273,6 +1270,8 @@ void Engine::prepare_multi() {
   cuda_check(cudaMemcpy(d_iaf_blk0_, blk0.data(), blk0.size() * sizeof(int), cudaMemcpyHostToDevice), "iaf table");
   cuda_check(cudaMemcpy(d_iaf_first_, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice),
              "iaf table");
+  iaf_tab_valid_ = true;
+  iaf_tab_seed_ = kernel_seed;
 }
 
 // The persistent step loop serves networks whose only neurons are iaf_psc_exp groups
@@ -1289,10 +1288,11 @@ void Engine::set_persistent(int on) {
 // then two short dependent launches otherwise (ngpu_persist.cu has both times).  With longer
 // minimum delays the per-batch kernels spread their launches over several steps and need no
 // barrier per step (3.5 us a step at 15-step batches, 12,500 neurons, 42k events a step).
-// A call costs a table upload, the first step's delivery from the ring and an extra barrier:
-// calls of 1, 2, 4, 8 and 16 steps took 78, 81, 84, 99 and 123 us on the microcircuit at a tenth
-// of its size (79, 85, 92, 110 and 142 us at full size) against 50, 63, 95, 149 and 267 us (54, 72,
-// 109, 184 and 337 us) per batch, so the line lies at four steps.  Networks whose draws have a
+// A call costs the first step's delivery from the ring, a gate and an extra barrier: calls of 1, 2, 3, 4, 5, 6
+// and 8 steps of 1000 neurons took 50, 53, 56, 59, 61, 65 and 70 us against 44, 51, 58, 66, 72, 80 and 94 us per
+// batch, of 100 neurons 49, 52, 56, 57, 58, 61 and 65 against 42, 48, 52, 58, 64, 70 and 80, of the microcircuit at
+// full size 55, 59, 64, 69, 74, 78 and 87 against 51, 65, 78, 92, 106, 121 and 148: the line lies at four steps.
+// Networks whose draws have a
 // kernel of their own (poisson_split) stay with the per-batch kernels: 8000 neurons of 2 / 4 / 10
 // generators each, loop 4.0 / 5.1 / 9.5 us per step, per batch 7.9 / 9.1 / 9.4.
 // A spiking neuron's edges of total delay one and two steps are delivered by its own block, two
@@ -1339,6 +1339,12 @@ bool Engine::iaf_only() const {
 // the launch was refused and the loop was the engine's own choice (the caller goes on per batch).
 // A launch whose blocks cannot all start runs no step and notes them in *h_skipped_.
 bool Engine::run_persistent(int steps) {
+  if (!h_skipped_) {   // (at the first launch: pinning costs 3 ms)
+    void *p = nullptr;
+    cuda_check(cudaHostAlloc(&p, sizeof(long long), cudaHostAllocMapped), "pinned counter");
+    h_skipped_ = (volatile long long *)p;
+    *h_skipped_ = 0;
+  }
   cuda_check(cudaMemsetAsync(d_bar_, 0, sizeof(GridBarrier), stream_), "barrier reset");
   const int r = loop_start_test == 1 ? -1 :
       launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_, steps, d_bar_,

@@ -202,3 +202,26 @@ def test_generators_take_no_place_in_the_loop():
     (got, launches), (want, _) = run(True), run(False)
     assert launches == 2
     assert want[0].sum() > 0 and all(np.array_equal(x, y) for x, y in zip(got, want))
+
+
+def test_table_of_the_loop_follows_the_settings():
+    """What the loop's argument table holds changes between calls: parameters (uniform ones become
+    arrays), recording, generator rates; against the per-batch kernels."""
+    def run(pers):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 400, 0.1, 2.0)
+        if not pers:
+            ngpu.SetPersistent(False)
+        rec = ngpu.CreateRecord("", ["V_m_rel"], [pops[0][1]], [0])
+        ngpu.Simulate(3.0)
+        ngpu.SetStatus(pops[1], "I_e", 350.0)
+        ngpu.Simulate(3.0)
+        ngpu.SetNeuronScalParam(pops[0][5], 3, "I_e", 420.0)
+        ngpu.Simulate(3.0)
+        ngpu.SetGraphSteps(50)
+        ngpu.Simulate(3.0)
+        assert (ngpu.GetLaunchMapping()["persistent"] == 1) == pers
+        return _state(ngpu, pops) + (np.asarray(ngpu.GetRecordData(rec)),)
+    got, want = run(True), run(False)
+    assert want[0].sum() > 20 and all(np.array_equal(x, y) for x, y in zip(got, want))
