@@ -399,6 +399,7 @@ class Engine {
   int *d_strag_cnt_ = nullptr;   // straggler counters, one per aeif group
   int n_strag_ = 0;
   int deliver_blocks_ = 148;
+  double mean_segment_ = 0.0;    // mean number of edges of a (source, delay) segment
   int deliver_long_ = 0;         // delivery: segments in parts, four edges in flight per lane
   int deliver_log2_parts_ = 0;   // parts per segment, by the mean segment length
   std::map<int, cudaGraphExec_t> graphs_;
@@ -520,7 +521,7 @@ int persistent_blocks(long long n_iaf, int dspan);
 long long persistent_own_edges(const long long *ev_off, int n_nodes, int dspan, unsigned long long *d_sum);
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
                           Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
-                          int barrier_extra, int gate_extra, cudaStream_t st);
+                          int barrier_extra, int gate_extra, double mean_segment, cudaStream_t st);
 int deliver_max_pairs();
 void pack_delivery_csr_noalloc(const int *src, const int *dly, const unsigned *target, const float *weight,
                                size_t n, int n_nodes, int dspan, unsigned long long *seg_off, EdgeW *edge,

@@ -83,8 +83,9 @@ __device__ __forceinline__ bool gate_wait(GridBarrier *bar) {
   return atomicCAS(&bar->state, (unsigned)GATE_WAIT, (unsigned)GATE_CLOSED) == GATE_OPEN;
 }
 
-// A segment's edges e, e + stride, ..., 128 of them at a time: four loads in flight per lane
-// before their reductions.  (Eight cost registers and spills, see PersShared.)
+// A segment's edges by LANES lanes: e, e + stride, ..., four of them LANES apart at a time, in flight
+// together before their reductions.  (Eight cost registers, and the kernel spills as it is.)
+template <int LANES>
 __device__ __forceinline__ void deliver_segment(const EdgeW *edge, double *acc, long long e0, int len, float height, int e,
                                                 int stride) {
   const uint2 *p = reinterpret_cast<const uint2 *>(edge) + e0;
@@ -92,10 +93,10 @@ __device__ __forceinline__ void deliver_segment(const EdgeW *edge, double *acc, 
     uint2 ew[4];
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      if (e + 32 * u < len) ew[u] = __ldg(p + e + 32 * u);
+      if (e + LANES * u < len) ew[u] = __ldg(p + e + LANES * u);
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      if (e + 32 * u < len) atomicAdd(&acc[ew[u].x], (double)__fmul_rn(height, __uint_as_float(ew[u].y)));
+      if (e + LANES * u < len) atomicAdd(&acc[ew[u].x], (double)__fmul_rn(height, __uint_as_float(ew[u].y)));
   }
 }
 
@@ -120,6 +121,8 @@ struct PersShared {
 
 __device__ __forceinline__ int slot_back(int rs, int d, int R) { return rs >= d ? rs - d : rs - d + R; }
 
+// LANES per segment of the delivery warps, by the mean segment's length (PERS_SHORT)
+template <int LANES>
 __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
     const DeliverArgs D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut so, const Clock *clk, int K,
     GridBarrier *bar, uint64_t seed, int extra, int gate_extra) {
@@ -160,18 +163,19 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
       carry += __shfl_sync(0xffffffffu, v, 31);
     }
   };
+  const int sub = lane & (LANES - 1);
   auto deliver_entry = [&](int sl, int j, int dd, double *acc) {
     const int2 sp = __ldcg(D.ring + (size_t)sl * D.cap + j);
     const size_t key = (size_t)sp.x * D.dspan + dd;
     const long long e0 = __ldg(D.ev_off + key), e1 = __ldg(D.ev_off + key + 1);
-    deliver_segment(D.edge, acc, e0, (int)(e1 - e0), __int_as_float(sp.y), lane, 128);
-    if (lane == 0) atomicAdd(&S.nev, (unsigned long long)(e1 - e0));
+    deliver_segment<LANES>(D.edge, acc, e0, (int)(e1 - e0), __int_as_float(sp.y), sub, 4 * LANES);
+    if (sub == 0) atomicAdd(&S.nev, (unsigned long long)(e1 - e0));
   };
-  // this block's share of those groups' segments, warp w of nw; consecutive ones go to
+  // this block's share of those groups' segments, thread t of nt; consecutive ones go to
   // different blocks
-  auto deliver_items = [&](int w, int nw, int rs0, int dd0, double *acc) {
+  auto deliver_items = [&](int t, int nt, int rs0, int dd0, double *acc) {
     const int np = D.dspan - dd0, total = s_pref[np];
-    for (int item = w * G + blockIdx.x; item < total; item += nw * G) {
+    for (int item = t / LANES * G + blockIdx.x; item < total; item += nt / LANES * G) {
       int a = 0, b = np;                // pair with s_pref[p] <= item < s_pref[p+1]
       while (b - a > 1) {
         const int mid = (a + b) >> 1;
@@ -195,10 +199,10 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
     if (!s_ok[0]) return;
     if (warp == 0) scan_counts(D.dspan);
     __syncthreads();
-    deliver_items(warp, PERS_THREADS / 32, rs0, 0, D.acc + (size_t)as * D.slot_stride);
+    deliver_items(tid, PERS_THREADS, rs0, 0, D.acc + (size_t)as * D.slot_stride);
     if (g1 >= 0 && K > 1 && t1 - 1 >= 1) {
       const int c = min(__ldcg(D.ring_cnt + rs0), D.cap);
-      for (int j = warp * G + blockIdx.x; j < c; j += (PERS_THREADS / 32) * G)
+      for (int j = tid / LANES * G + blockIdx.x; j < c; j += PERS_THREADS / LANES * G)
         deliver_entry(rs0, j, g1, D.acc + (size_t)((as + 1) % PERS_SLOTS) * D.slot_stride);
     }
     __syncthreads();
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
       nb_sync(NB_DELIVER, PERS_DELIVER);
       if (dw == 0) scan_counts(D.dspan - gd);
       nb_sync(NB_DELIVER, PERS_DELIVER);
-      deliver_items(dw, PERS_DELIVER / 32, rs, gd, D.acc + (size_t)as * D.slot_stride);
+      deliver_items(dt, PERS_DELIVER, rs, gd, D.acc + (size_t)as * D.slot_stride);
       nb_arrive(NB_DONE + ((k + 1) & 1), PERS_THREADS);
       nb_sync(NB_NEXT + (k & 1), PERS_THREADS);
       if (!s_ok[k & 1]) break;
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
       if (!last)
         for (int j = rwarp >> 1; j < ns; j += PERS_NEURON / 64) {
           const int o = S.own[j], len = S.len[o].x;
-          deliver_segment(D.edge, D.acc + (size_t)as1 * D.slot_stride, S.e0[o], len, 1.0f, half, 256);
+          deliver_segment<32>(D.edge, D.acc + (size_t)as1 * D.slot_stride, S.e0[o], len, 1.0f, half, 256);
           if (half == 0) atomicAdd(&S.nev, (unsigned long long)len);
         }
       nb_sync(NB_DONE + par, PERS_THREADS);
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(PERS_THREADS, 1) persistent_iaf_kernel(
         for (int j = rwarp >> 1; j < ns; j += PERS_NEURON / 64) {
           const int o = S.own[j];
           const int2 len = S.len[o];
-          deliver_segment(D.edge, D.acc + (size_t)((as + 2) % PERS_SLOTS) * D.slot_stride, S.e0[o] + len.x, len.y, 1.0f,
+          deliver_segment<32>(D.edge, D.acc + (size_t)((as + 2) % PERS_SLOTS) * D.slot_stride, S.e0[o] + len.x, len.y, 1.0f,
                           half, 256);
           if (half == 0) atomicAdd(&S.nev, (unsigned long long)len.y);
         }
@@ -449,18 +453,29 @@ int persistent_blocks(long long n_iaf, int dspan) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   if (dspan > PERS_MAX_SPAN || n_iaf > (long long)n_sm * PERS_NEURON) return 0;
-  if (cudaFuncSetAttribute(persistent_iaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersShared)) !=
-      cudaSuccess)
-    return 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_iaf_kernel, PERS_THREADS, sizeof(PersShared));
-  return per_sm >= 1 ? n_sm : 0;
+  for (auto *kernel : {persistent_iaf_kernel<8>, persistent_iaf_kernel<32>}) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersShared)) != cudaSuccess)
+      return 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, PERS_THREADS, sizeof(PersShared));
+    if (per_sm < 1) return 0;
+  }
+  return n_sm;
 }
+
+// A warp of the delivery warps serves one segment, or four short ones side by side: what a segment
+// costs there is its chain of four dependent loads, whatever its length.  us per step, a warp / eight lanes a segment, 70,000
+// neurons of 29 delay groups and 550 spikes a step: 7 edges a segment 23.0 / 10.2, 34 edges 26.3 /
+// 13.4; 40,000 neurons, 315 spikes, 50 edges 16.0 / 9.6; 20,000 of 10 groups, 160 spikes, 60 edges
+// 3.9 / 3.8, but 100 edges 4.2 / 5.0, and the layered microcircuit (130 edges) 3.6 / 7.8 at a tenth of
+// its size, 4.6 / 10.5 at full size.
+constexpr double PERS_SHORT = 64.0;
 
 // Cooperative launch of the persistent loop over `steps` steps, then the clock; the number of
 // launches, or -1 where the cooperative launch is refused.
 int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *first, int ngroups, const SpikeOut &so,
                           Clock *clk, int steps, GridBarrier *bar, long long *skipped, uint64_t seed, int nblocks,
-                          int barrier_extra, int gate_extra, cudaStream_t st) {
+                          int barrier_extra, int gate_extra, double mean_segment, cudaStream_t st) {
+  void *kernel = mean_segment <= PERS_SHORT ? (void *)persistent_iaf_kernel<8> : (void *)persistent_iaf_kernel<32>;
   DeliverArgs d = D;
   const IafArgs *t = tab;
   const int *f = first;
@@ -472,9 +487,7 @@ int launch_persistent_iaf(const DeliverArgs &D, const IafArgs *tab, const int *f
   uint64_t sd = seed;
   int x = barrier_extra, gx = gate_extra;
   void *args[] = {&d, &t, &f, &ng, &s, &c, &k, &b, &sd, &x, &gx};
-  if (cudaLaunchCooperativeKernel((void *)persistent_iaf_kernel, dim3(nblocks), dim3(PERS_THREADS), args,
-                                  sizeof(PersShared), st) !=
-      cudaSuccess)
+  if (cudaLaunchCooperativeKernel(kernel, dim3(nblocks), dim3(PERS_THREADS), args, sizeof(PersShared), st) != cudaSuccess)
     return -1;
   persistent_advance_kernel<<<1, 1, 0, st>>>(clk, steps, bar, skipped);
   return 2;

@@ -483,7 +483,7 @@ void Engine::calibrate() {
   d_clk_ = dalloc<Clock>(1);
   cuda_check(cudaMemset(d_clk_, 0, sizeof(Clock)), "clock");
   deliver_blocks_ = std::max(1, std::min(148 * 8, (n_src_out + 63) / 64));
-  const double mean_len = n_src_out > 0 ? (double)n_edge_dev_ / ((double)n_src_out * dspan_) : 0.0;
+  mean_segment_ = n_src_out > 0 ? (double)n_edge_dev_ / ((double)n_src_out * dspan_) : 0.0;
   // With slots of many megabytes fewer work items in flight keep fewer arrival steps open, so that
   // the reductions stay in L2.  Blocks 296 / 592 / 1184, ms: 500k AdEx (8 MB a slot, 30 ms) 12.0 /
   // 11.0 / 11.1, 1M (16 MB, 50 ms) 34.6 / 31.8 / 34.7, 2.8M ensemble (45 MB, 20 ms) 24.6 / 26.9 /
@@ -491,7 +491,7 @@ void Engine::calibrate() {
   // for a few reductions, need all of them: 1M iaf_psc_exp neurons, 592 / 1184, ms per 10 ms,
   // segments of 200 edges 3.49 / 3.88, 90 edges 7.46 / 8.22, 9 edges 4.55 / 3.86, one edge or none
   // 21.6 / 13.0; and short batches have few arrival steps anyway (100 edges, one step 4.08 / 3.88).
-  while (mean_len >= 32.0 && batch_ >= 8 && deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184)
+  while (mean_segment_ >= 32.0 && batch_ >= 8 && deliver_blocks_ > 296 && (double)n_acc_ * sizeof(double) * deliver_blocks_ > 12e6 * 1184)
     deliver_blocks_ /= 2;
   // Long (source, delay) segments are delivered in parts of about 128 edges (the four loads that a
   // 32-lane group has in flight), so that a batch's few spikes fill the GPU: 12,500 neurons with
@@ -502,10 +502,10 @@ void Engine::calibrate() {
   // 166 411 / 430; but 16 MB, 67 474 / 441; 24 MB, 64 231 / 219 and 300 1133 / 1075; 32 MB, 90 1539 /
   // 1499; 144 MB, 300 2576 / 2483.  By length: 0.1 MB, 64 edges 144 / 148; 0.5 MB, 42 edges 206 / 212;
   // but 0.3 MB, 18 edges 236 / 229; 1 MB, 7 edges 1537 / 1321.
-  deliver_long_ = mean_len >= 32.0 && (double)n_acc_ * sizeof(double) * batch_ <= 12e6;
+  deliver_long_ = mean_segment_ >= 32.0 && (double)n_acc_ * sizeof(double) * batch_ <= 12e6;
   deliver_log2_parts_ = 0;
   if (deliver_long_)
-    while (deliver_log2_parts_ < 4 && mean_len > (128 << deliver_log2_parts_)) deliver_log2_parts_++;
+    while (deliver_log2_parts_ < 4 && mean_segment_ > (128 << deliver_log2_parts_)) deliver_log2_parts_++;
   if (plastic_) build_plastic(pl_edge, pl_key, pl_rank);
   // ---- dendritic delays: the reverse ring (plastic networks only; src/spike_buffer.cu:162-317)
   if (plastic_) {
@@ -1349,7 +1349,7 @@ bool Engine::run_persistent(int steps) {
   const int r = loop_start_test == 1 ? -1 :
       launch_persistent_iaf(deliver_args(), d_iaf_tab_, d_iaf_first_, n_iaf_multi_, spike_out(), d_clk_, steps, d_bar_,
                             (long long *)h_skipped_, kernel_seed, pers_blocks_, barrier_extra, loop_start_test == 2,
-                            stream_);
+                            mean_segment_, stream_);
   if (r < 0 && persistent != 1) {
     cudaGetLastError();
     loop_failed_ = true;

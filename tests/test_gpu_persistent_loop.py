@@ -225,3 +225,51 @@ def test_table_of_the_loop_follows_the_settings():
         return _state(ngpu, pops) + (np.asarray(ngpu.GetRecordData(rec)),)
     got, want = run(True), run(False)
     assert want[0].sum() > 20 and all(np.array_equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("k,lo,hi", [(62, 0.1, 0.1), (66, 0.1, 0.1), (500, 0.1, 1.0), (700, 0.1, 1.0), (130, 0.3, 0.3), (9, 0.1, 1.7)])
+def test_segment_lengths_match_oracle(k, lo, hi):
+    """Mean segments around 64 edges, where the delivery warps go from eight lanes a segment to a
+    warp, and longer ones than a warp has in flight (128 edges)."""
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 8)
+        n = api.Create("iaf_psc_exp", 300)
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 12000.0)
+        api.Connect(pg, n, {"rule": "all_to_all"}, {"weight": 45.0, "delay": 1.0, "receptor": 0})
+        api.ConnectFixedIndegreeGPU(n, n, k, 60.0 / k, lo, hi, receptor=0, seed=2)
+        api.ActivateSpikeCount(n)
+        api.Simulate(25.0)
+        return _state(api, [n])
+    ngpu.SetPersistent(True)
+    got = run(ngpu)
+    o = orc.Oracle()
+    want = run(o)
+    assert ngpu.GetLaunchMapping()["persistent"] == 1
+    assert want[0].sum() > 50 and all(np.array_equal(x, y) for x, y in zip(got, want))
+    assert ngpu.GetStats()["n_events"] == o.NEvents()
+
+
+def test_generators_of_all_kinds_match_oracle():
+    """One generator on receptor 1, one with a mean count above ten, one that is off at first, several
+    per neuron; recorded spike times."""
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 12)
+        n = api.Create("iaf_psc_exp", 120)
+        pg = api.Create("poisson_generator", 5)
+        for i, (rate, receptor, w) in enumerate([(9000.0, 0, 50.0), (9000.0, 1, 50.0), (130000.0, 1, 4.0), (9000.0, 0, 55.0),
+                                                 (4000.0, 0, 60.0)]):
+            api.SetStatus([pg[i]], "rate", rate)
+            api.Connect([pg[i]], n[24 * i:24 * i + 24], {"rule": "all_to_all"}, {"weight": w, "delay": 1.0, "receptor": receptor})
+        api.SetStatus([pg[3]], {"start": 4.0})
+        api.Connect([pg[0]], n[96:120], {"rule": "all_to_all"}, {"weight": 30.0, "delay": 0.5, "receptor": 1})
+        api.ConnectFixedIndegreeGPU(n, n, 20, 8.0, 0.1, 1.0, receptor=0, seed=2)
+        api.ActivateSpikeCount(n)
+        api.ActivateRecSpikeTimes(n, 200)
+        api.Simulate(17.0)
+        api.Simulate(9.0)
+        return _state(api, [n]) + (np.concatenate([np.asarray(t, dtype=np.float32) for t in api.GetRecSpikeTimes(n)]),)
+    ngpu.SetPersistent(True)
+    got, want = run(ngpu), run(orc.Oracle())
+    assert ngpu.GetLaunchMapping()["persistent"] == 1
+    assert want[0].sum() > 100 and all(np.array_equal(x, y) for x, y in zip(got, want))
