@@ -895,7 +895,7 @@ PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
 }
 
 // Launch mapping of a group's aeif update where the caller set none.
-// A group that is resident at once in the kernel without a register cap (aeif_resident: 66k
+// A group that is resident at once in the kernel without a register cap (aeif_resident: 57k
 // neurons for the two-port conductance model) loses nothing by letting a spiking neuron finish its
 // 40 to 60 sub-steps in its own warp; handing it to the straggler kernel would only add a launch to
 // the chain that sets the batch's length.  A larger group needs the block slots: neurons beyond a
@@ -910,15 +910,18 @@ PoissonMultiArgs Engine::poisson_multi_args(Group &g) {
 // There a batch's stragglers are worth a hand-off at every size, and a thin warp's loads fill a line
 // each: 128-thread blocks of full warps, hand-off after M + 4.  beta with 6 ports, us per 10 ms, so /
 // by the rules for fewer ports: 1000 neurons 2086 / 5342 (quiet), 11,010 / 11,302 (active), 30,000
-// 20,567 / 28,174.  The same for one port in one-step batches beyond the resident neurons: 150,000
+// 20,567 / 28,174.  (One-step batches of groups that are resident at once, 37,888 neurons, do without
+// the second launch: 17,000 active neurons 47.7 ms, 68.8 with the hand-off; 100,000 142 / 121.)  The
+// same for one port in one-step batches beyond the resident neurons: 150,000
 // active beta neurons 9.1 ms per 10 ms, 13.1 without a hand-off (quiet 1.34, 1.46).
 void Engine::aeif_mapping(const Group &g, AeifArgs &A) const {
   const bool any_ports = g.nport > 4;
-  const bool late = any_ports || (g.nport == 1 && batch_ == 1 && A.hi - A.lo > g.resident);
-  const bool hand_off = !late && A.hi - A.lo > (batch_ == 1 ? 3 * g.resident : g.resident);
+  const bool late = any_ports ? batch_ > 1 || A.hi - A.lo > 148 * 256
+                              : g.nport == 1 && batch_ == 1 && A.hi - A.lo > g.resident;
+  const bool hand_off = !late && !any_ports && A.hi - A.lo > (batch_ == 1 ? 3 * g.resident : g.resident);
   const int budget = rk5_budget >= 0 ? rk5_budget : late ? 4 : (hand_off ? 1 : 0);
   A.budget = budget > 0 ? batch_ + budget : 0;
-  A.threads = update_threads > 0 ? update_threads : late ? 128 : 64;
+  A.threads = update_threads > 0 ? update_threads : late || any_ports ? 128 : 64;
   A.occupancy = update_occupancy >= 0 ? update_occupancy : (hand_off ? 2 : 0);
   A.trial_iter = update_trial_iter >= 0 ? update_trial_iter : (hand_off ? 1 : 0);
   // The lanes of a warp wait for each other in every step (rejected trials, the network's
@@ -1319,7 +1322,8 @@ bool Engine::use_loop(long long steps) const {
   return persistent > 0 && persistent_eligible();
 }
 
-// Delivery at emission serves the same networks as the persistent loop.
+// Delivery at emission serves the networks of the persistent loop, of any size and with any number of
+// delay groups.
 bool Engine::push_eligible() const { return iaf_only(); }
 
 // iaf_psc_exp groups only (their spikes have height 1 and their kernel is the only spike

@@ -122,7 +122,7 @@ def test_long_first_segments_stay_with_the_per_batch_kernels(k, hi, loop):
         assert np.array_equal(got[1], other[1]) and np.array_equal(got[2], other[2])
 
 
-@pytest.mark.parametrize("ports,n,delay,want", [(5, 60, 1.0, (128, 0, 0, 4)), (20, 33, 0.3, (128, 0, 0, 4)),
+@pytest.mark.parametrize("ports,n,delay,want", [(5, 60, 1.0, (128, 0, 0, 4)), (20, 33, 0.3, (128, 0, 0, 4)), (6, 45, 0.1, (128, 0, 0, 0)),
                                                 (1, 60, 0.1, (64, 0, 0, 0)), (1, 130000, 0.1, (128, 0, 0, 4))])
 def test_one_port_and_any_number_of_ports(ports, n, delay, want):
     """The mappings of their own, against the oracle where that is quick."""
@@ -146,3 +146,26 @@ def test_one_port_and_any_number_of_ports(ports, n, delay, want):
     if n < 1000:
         co, vo = run(orc.Oracle())
         assert co.sum() > 0 and np.array_equal(c, co) and np.array_equal(v, vo)
+
+
+@pytest.mark.parametrize("n,want", [(50000, (64, 0, 0, 0)), (76000, (64, 2, 1, 1))])
+def test_both_sides_of_the_resident_neurons_match_oracle(n, want):
+    """Groups below and above the neurons that are resident at once (56,832 for two ports): no
+    hand-off, and the capped kernel with the straggler kernel."""
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 6)
+        neuron = api.Create("aeif_cond_beta_multisynapse", n, 2)
+        api.SetStatus(neuron, {"E_rev": [0.0, -85.0]})
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 8000.0)
+        api.Connect(pg, neuron, {"rule": "all_to_all"}, {"weight": 2.0, "delay": 0.1, "receptor": 0})
+        api.ConnectFixedIndegreeGPU(neuron, neuron, 2, 0.3, 1.0, 1.5, receptor=1, seed=5)
+        api.ActivateSpikeCount(neuron)
+        api.Simulate(6.0)
+        return (np.asarray(api.GetStatus(neuron, "spike_count")).ravel(),
+                np.asarray(api.GetStatus(neuron, "V_m"), dtype=np.float32).ravel())
+    c, v = run(ngpu)
+    m = ngpu.GetLaunchMapping()
+    assert (m["update_threads"], m["update_occupancy"], m["update_trial_iter"], m["rk5_budget"]) == want
+    co, vo = run(orc.Oracle())
+    assert co.sum() > 1000 and np.array_equal(c, co) and np.array_equal(v, vo)
