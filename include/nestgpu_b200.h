@@ -337,7 +337,8 @@ int NGPU_SetGraphSteps(int n);
    launch (the minimum delay in steps + 1, at most 32 and at most the batch_max setting). */
 int NGPU_GetBatchLength(void);
 
-/* Threads per block of the aeif update kernel (64, 128 or 256; without a call 64). */
+/* Threads per block of the aeif update kernel (64, 128 or 256; without a call chosen from the
+   group's ports and size). */
 int NGPU_SetUpdateThreads(int n);
 /* 1: use the register-capped variant of the aeif update kernel (three 256-thread blocks per
    SM, more warps in flight, a few register spills); 2: with the trial-per-iteration update

@@ -138,7 +138,8 @@ class Engine {
                                   // takes over (0: it never does; -1: by aeif_mapping)
   int deliver_blocks_req = 0;     // delivery grid size (0: from the number of spiking sources)
   int batch_max = MAX_BATCH;      // upper bound of the time-batch length (1: step by step)
-  int update_threads = 0;         // threads per block of the aeif update kernel (64, 128, 256; 0: 64)
+  int update_threads = 0;         // threads per block of the aeif update kernel (64, 128, 256; 0: by
+                                  // aeif_mapping)
   int deliver_group = 32;         // lanes per delivery work item (8, 16, 32)
   int deliver_aggregate = 0;      // 1: warp-aggregated reductions (with 32-lane work items)
   int deliver_prefetch = 0;       // 1: delivery loads the next work item's segment ahead

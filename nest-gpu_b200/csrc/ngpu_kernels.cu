@@ -358,13 +358,11 @@ __global__ void spike_gen_batch_kernel(const SpikeGenArgs A, const SpikeOut so, 
 // poiss_gen draws of a group in which some neuron has several generators: one thread per
 // (edge, block of four time indices) adds the edge's draws of the batch into the accumulator
 // slots that the update kernel folds.  The draws are those of poisson_draw: the same counters,
-// one Philox call per four steps.  Bound by integer issue (Philox, about 100 instructions per
-// four draws); drawn inside the update kernel instead, a neuron's edges were one serial chain
-// in one thread: 1000 neurons x 400 generators at 20 Hz, 15-step batches, took 8.9 ms per batch
-// in the batch and straggler kernels, and 20 ms of that network 127.0 ms against 1.98 ms now.
-// A neuron with one edge keeps the draw in its update kernel (PoissonCache: no pass over
-// memory); the line lies at two edges because from there on the update kernel would redo the
-// Philox call and exp(-lambda) of every edge in every step.
+// one Philox call (about 100 integer instructions) per four steps.  Drawn inside the update kernel
+// instead, a neuron's edges were one serial chain in one thread: 1000 neurons x 400 generators at
+// 20 Hz, 15-step batches, took 8.9 ms per batch in the batch and straggler kernels, and 20 ms of that
+// network 127.0 ms against 1.98 ms now.  Engine::poisson_line has the number of generators from
+// which the draws move here.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) poisson_multi_kernel(const PoissonMultiArgs A, const Clock *clk, int k0, int M) {
   pdl_enter();

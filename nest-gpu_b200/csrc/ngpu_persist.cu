@@ -17,7 +17,8 @@ namespace ngpu {
 // spikes in the ring, add their edges that arrive in step s + 2, draw the Poisson input; wait;
 // fold the input of step s.  Its delivery warps meanwhile add the block's share of all other
 // edges that arrive in step s + 1: spikes of steps <= s - 2, which were filed before barrier
-// s - 1, a warp per (spike, delay) segment, spread over all blocks.  They have from barrier s - 1
+// s - 1, a warp or, where segments are short, eight lanes per (spike, delay) segment, spread over all
+// blocks.  They have from barrier s - 1
 // until the block arrives at barrier s + 1, so their chain of four dependent loads stays off the
 // critical path, which is: fold, update, the own spikes' first edges, the fence behind their
 // reductions, and the barrier's round trip through L2.

@@ -100,3 +100,32 @@ def test_delivery_forms_match_oracle(n, k, hi, group, prefetch):
     co, vo = run(o)
     assert co.sum() > 0 and np.array_equal(c, co) and np.array_equal(v, vo)
     assert ngpu.GetStats()["n_events"] == o.NEvents()
+
+
+@pytest.mark.parametrize("n", [1036, 1037])
+def test_step_model_in_thin_warps_matches_oracle(n):
+    """The step model proposing in groups of one and of two neurons per warp."""
+    from test_oracle_learn import random_params
+    p = random_params(21)
+    p[1461], p[1462] = np.float32(np.log(0.02)), 0.5
+
+    def run(api):
+        api.SetKernelStatus("rnd_seed", 11)
+        neuron = api.Create("aeif_cond_beta_multisynapse", n, 4)
+        api.SetStatus(neuron, {"E_rev": [0.0, 0.0, -85.0, -85.0]})
+        pg = api.Create("poisson_generator")
+        api.SetStatus(pg, "rate", 4000.0)
+        api.Connect(pg, neuron, {"rule": "all_to_all"}, {"weight": 1.5, "delay": 1.0, "receptor": 0})
+        api.ConnectFixedIndegreeGPU(neuron, neuron, 10, 0.1, 1.5, 1.5, receptor=1, seed=3)
+        api.ActivateSpikeCount(neuron)
+        if api is ngpu:
+            ngpu.StepModelSet(p)
+            ngpu.StepModelEnable(True)
+        else:
+            api.StepModelSet(p, enable=True)
+        api.Simulate(12.0)
+        return (np.asarray(api.GetStatus(neuron, "spike_count")).ravel(),
+                np.asarray(api.GetStatus(neuron, "V_m"), dtype=np.float32).ravel())
+    c, v = run(ngpu)
+    co, vo = run(orc.Oracle())
+    assert co.sum() > 0 and np.array_equal(c, co) and np.array_equal(v, vo)

@@ -85,8 +85,8 @@ def test_capacity_and_what_lies_beyond_it(n, hi, loop):
 
 
 def test_turns_between_the_forms():
-    """Persistent calls, per-batch calls, single steps and short calls of the automatic choice,
-    spikes in flight at every change, give what the per-batch kernels alone give."""
+    """Forced persistent calls, per-batch calls and single steps, spikes in flight at every change,
+    give what the per-batch kernels alone give."""
     def run(modes):
         ngpu.Reset()
         ngpu.SetVerbosityLevel(0)
@@ -105,15 +105,38 @@ def test_turns_between_the_forms():
         assert all(np.array_equal(x, y) for x, y in zip(run(modes), want))
 
 
+def test_automatic_choice_by_call_length():
+    """Without a call to SetPersistent: the loop from four steps a call on, shorter calls and single
+    steps per batch, on the same ring and accumulators; what the per-batch kernels alone give."""
+    def run(auto):
+        ngpu.Reset()
+        ngpu.SetVerbosityLevel(0)
+        pops = _net(ngpu, 500, 0.1, 2.9)
+        if not auto:
+            ngpu.SetPersistent(False)
+        loops = []
+        for t in (4.0, 0.3, 0.4, 1.1, 0.2, 0.1, 5.0, 0.3, 2.0):
+            loops.append(_count_launches(lambda: ngpu.Simulate(t)) == 2)
+            ngpu.SimulationStep()
+            ngpu.EndSimulation()
+        return _state(ngpu, pops) + (ngpu.GetStats()["n_events"],), loops
+    (got, loops), (want, none) = run(True), run(False)
+    assert loops == [True, False, True, True, False, False, True, False, True] and not any(none)
+    assert want[0].sum() > 50 and all(np.array_equal(x, y) for x, y in zip(got, want))
+
+
 def test_two_networks_in_two_threads():
     """Two host threads run a network each at the same time (one engine per thread): their
-    persistent launches share the GPU and the results are those of a network alone."""
+    persistent launches share the GPU and the results are those of each network alone in the
+    per-batch kernels."""
     import threading
 
     def run(out, key):
         ngpu.SetOnException(1)     # error handling is per thread
         ngpu.SetVerbosityLevel(0)
         pops = _net(ngpu, 800 + key, 0.1, 2.0)
+        if out is alone:
+            ngpu.SetPersistent(False)
         for _ in range(20):
             ngpu.Simulate(5.0)
         out[key] = _state(ngpu, pops)
